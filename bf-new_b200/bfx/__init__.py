@@ -637,6 +637,11 @@ class Workspace:
         registers per thread for the persistent kernel."""
         _check(load().bfx_set_register_budget(self._h, u32(registers)))
 
+    def set_resident_nets(self, mode: int):
+        """1 (default): frontier lanes that fit a thread-block cluster's shared memory are relaxed there;
+        0: every lane takes the grid-wide kernels."""
+        _check(load().bfx_set_resident_nets(self._h, u32(mode)))
+
     def set_chunk_pairs(self, mode: int):
         """Chunked layout: 0 work list, 1 (vertex, lane) pair per thread (persistent control)."""
         _check(load().bfx_set_chunk_pairs(self._h, u32(mode)))

@@ -35,6 +35,7 @@
 #include "bfx_internal.hpp"
 #include "device_common.cuh"
 #include "engine_types.cuh"
+#include "resident.cuh"
 
 #include <cuda_runtime.h>
 
@@ -290,7 +291,9 @@ __global__ void seed_kernel(LaunchParams p, const u32* src_base) {
     B.dist[0][(static_cast<u64>(cv) << B.shift) + lane] = dev::kSourceWord;
     const u32 eng = engine_of(p, b);
     if (eng == BFX_ENGINE_JACOBI_PULL) B.dist[1][(static_cast<u64>(cv) << B.shift) + lane] = dev::kSourceWord;
-    if (eng == BFX_ENGINE_FRONTIER_PUSH && p.flat >= 2u) {
+    if (eng == BFX_ENGINE_FRONTIER_PUSH && p.fit != nullptr && ((p.fit[b] >> lane) & 1u)) {
+      // relaxed by its own cluster (resident.cu), which finds its sources itself
+    } else if (eng == BFX_ENGINE_FRONTIER_PUSH && p.flat >= 2u) {
       // chunked / tiled frontier: pending lane, then the claim unit's bit;
       // the thread that sets the bit queues the unit
       atomicOr(&B.mask[0][cv], 1u << lane);
@@ -1175,6 +1178,7 @@ int bfx_resident_graph_upload(const bfx_device_graph_layout32* layout, int devic
     std::vector<uint4> csr(E), csc(E);
     std::vector<std::uint32_t> eid_src(E, 0U);
     std::vector<uint2> lrun(V);
+    std::vector<uint2> csr_row(V);
     bfx::parallel_for(V, 0, [&](std::uint64_t b, std::uint64_t e) {
       for (std::uint64_t v = b; v < e; ++v) {
         // own-tile run: rows are ordered by destination tile, so the edges
@@ -1187,6 +1191,7 @@ int bfx_resident_graph_upload(const bfx_device_graph_layout32* layout, int devic
           }
         }
         lrun[v] = make_uint2(lb, lc);
+        csr_row[v] = make_uint2(L.csr_row_offsets[v], L.csr_row_offsets[v + 1] - L.csr_row_offsets[v]);
         for (std::uint32_t p = L.csr_row_offsets[v]; p < L.csr_row_offsets[v + 1]; ++p) {
           const std::uint32_t d = L.csr_destinations[p];
           std::uint32_t wb;
@@ -1211,7 +1216,8 @@ int bfx_resident_graph_upload(const bfx_device_graph_layout32* layout, int devic
     const size_t o_eid_src = bfx::align256(o_csc + size_t{E} * 16);
     const size_t o_lrun = bfx::align256(o_eid_src + size_t{E} * 4);
     const size_t o_toff = bfx::align256(o_lrun + size_t{V} * 8);
-    const size_t total = bfx::align256(o_toff + (size_t{T} + 1) * 4);
+    const size_t o_row = bfx::align256(o_toff + (size_t{T} + 1) * 4);
+    const size_t total = bfx::align256(o_row + size_t{V} * 8);
     G->mem.reserve(total, device);
     char* base = static_cast<char*>(G->mem.ptr);
     BFX_CUDA(cudaMemcpy(base + o_owner, L.owner_tiles, size_t{V} * 4, cudaMemcpyHostToDevice));
@@ -1222,6 +1228,7 @@ int bfx_resident_graph_upload(const bfx_device_graph_layout32* layout, int devic
     BFX_CUDA(cudaMemcpy(base + o_eid_src, eid_src.data(), size_t{E} * 4, cudaMemcpyHostToDevice));
     BFX_CUDA(cudaMemcpy(base + o_lrun, lrun.data(), size_t{V} * 8, cudaMemcpyHostToDevice));
     BFX_CUDA(cudaMemcpy(base + o_toff, G->tile_vertex_offsets.data(), (size_t{T} + 1) * 4, cudaMemcpyHostToDevice));
+    BFX_CUDA(cudaMemcpy(base + o_row, csr_row.data(), size_t{V} * 8, cudaMemcpyHostToDevice));
     double wsum = 0.0;
     for (std::uint32_t e = 0; e < E; ++e) wsum += L.csr_weights[e];
     G->mean_weight = E ? wsum / E : 0.0;
@@ -1236,6 +1243,7 @@ int bfx_resident_graph_upload(const bfx_device_graph_layout32* layout, int devic
     G->g.eid_src = reinterpret_cast<const std::uint32_t*>(base + o_eid_src);
     G->g.lrun = reinterpret_cast<const uint2*>(base + o_lrun);
     G->g.tile_off = reinterpret_cast<const std::uint32_t*>(base + o_toff);
+    G->g.csr_row = reinterpret_cast<const uint2*>(base + o_row);
     G->bytes = total;
     {
       const std::uint32_t size0 = G->tile_vertex_offsets[1] - G->tile_vertex_offsets[0];
@@ -1250,6 +1258,14 @@ int bfx_resident_graph_upload(const bfx_device_graph_layout32* layout, int devic
         shift = 5;
       }
       G->tile_shift = shift;
+      const std::uint32_t words = (size0 + 31U) / 32U;
+      bool same = words != 0U;
+      for (std::uint32_t t = 0; t < T && same; ++t) {
+        same = (G->tile_vertex_offsets[t + 1] - G->tile_vertex_offsets[t] + 31U) / 32U == words;
+      }
+      G->resident_shapes = bfx::resident_shapes();
+      G->word_whole = same && words <= 32U && (words & (words - 1U)) == 0U;
+      if (G->word_whole) G->word_run = static_cast<std::uint32_t>(__builtin_ctz(words));
     }
     *out = G.release();
   });
@@ -1297,6 +1313,7 @@ int bfx_workspace_destroy(bfx_workspace* ws) {
     cudaSetDevice(ws->graph->device);
     if (ws->stream) cudaStreamSynchronize(ws->stream);
     if (ws->chunk_exec) cudaGraphExecDestroy(ws->chunk_exec);
+    bfx::resident_release(ws);
     for (auto& e : ws->ev) {
       if (e) cudaEventDestroy(e);
     }
@@ -1341,14 +1358,18 @@ struct DescArrays {
 // pile state, chunk bitmaps, row tables) and the tile tables (one dense
 // {lane mask, compact bias} table per batch).  Fills ws->batches with device
 // pointers, the staging header (records, prefixes) and the launch
-// parameters; the caller writes the description arrays and uploads.
+// parameters; the caller writes the description arrays and uploads.  `nets`:
+// one entry per valid lane, sorted and reduced to those that fit a cluster.
 struct Layout {
   size_t o_up, meta_total;
   std::vector<DescArrays> arrays;
 };
 
-Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector<BatchSizes>& sz) {
+Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector<BatchSizes>& sz,
+                       std::vector<ResidentNet>& nets) {
   const DGraph& g = ws->graph->g;
+  std::vector<u32> fit(count, 0u);
+  resident_select(ws, nets, fit);
   const size_t o_batch = 0;
   const size_t o_ctl = align256(o_batch + count * sizeof(DBatch));
   const size_t o_run = align256(o_ctl + count * sizeof(DCtl));
@@ -1356,8 +1377,10 @@ Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector
   const size_t o_sbase = align256(o_ubase + (count + 1) * 4);
   const size_t o_status = align256(o_sbase + (count + 1) * 4);
   const size_t o_ctrl = align256(o_status + count * sizeof(bfx_device_run_status));
+  const size_t o_fit = align256(o_ctrl + count * sizeof(bfx_device_controller));
+  const size_t o_nets = align256(o_fit + count * 4);
   Layout L;
-  L.o_up = align256(o_ctrl + count * sizeof(bfx_device_controller));
+  L.o_up = align256(o_nets + nets.size() * sizeof(ResidentNet));
   L.arrays.resize(count);
   size_t up = L.o_up;
   for (std::uint32_t b = 0; b < count; ++b) {
@@ -1462,6 +1485,12 @@ Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector
   ubase[count] = static_cast<std::uint32_t>(usum);
   sbase[count] = static_cast<std::uint32_t>(ssum);
   std::memcpy(hb + o_batch, ws->batches.data(), count * sizeof(DBatch));
+  std::memcpy(hb + o_fit, fit.data(), count * 4);
+  if (!nets.empty()) std::memcpy(hb + o_nets, nets.data(), nets.size() * sizeof(ResidentNet));
+  ws->fit.swap(fit);
+  ws->nets.swap(nets);
+  ws->d_fit = reinterpret_cast<const u32*>(db + o_fit);
+  ws->d_nets = reinterpret_cast<const ResidentNet*>(db + o_nets);
   ws->nb = count;
   ws->src_total = ssum;
   ws->params = LaunchParams{};
@@ -1494,6 +1523,7 @@ int bfx_prepare_batches(bfx_workspace* ws, uint32_t count, const bfx_batch_descr
     // Validate descriptions (validate_batch_device_description,
     // include/bfnew/batch_layout.hpp:176-199) and size everything.
     std::vector<bfx::BatchSizes> sz(count);
+    std::vector<bfx::ResidentNet> nets;
     for (std::uint32_t b = 0; b < count; ++b) {
       const bfx_batch_description& d = batches[b];
       const std::uint32_t W = d.lane_width;
@@ -1518,6 +1548,9 @@ int bfx_prepare_batches(bfx_workspace* ws, uint32_t count, const bfx_batch_descr
       bfx::require(Tg == 0 || d.targets, "null targets");
       bfx::require(d.range_count == d.union_tile_count, "one vertex range per union tile is required");
       std::uint64_t U = 0;
+      // per lane: selected tiles and the 32-vertex words they fill; [32]: of
+      // the tiles that every valid lane selects
+      std::uint32_t words[33] = {}, tiles[33] = {};
       for (std::uint32_t i = 0; i < d.union_tile_count; ++i) {
         const std::uint32_t t = d.union_tiles[i];
         if (t >= g.T) throw std::out_of_range("union tile out of range");
@@ -1527,6 +1560,20 @@ int bfx_prepare_batches(bfx_workspace* ws, uint32_t count, const bfx_batch_descr
         bfx::require(r.lane_mask == d.tile_lane_masks[t] && r.lane_mask != 0 && (r.lane_mask & ~d.valid_lane_mask) == 0,
                      "invalid tile lane mask");
         U += r.end - r.begin;
+        const std::uint32_t w = (r.end - r.begin + 31U) / 32U;
+        for (std::uint32_t m = r.lane_mask == d.valid_lane_mask ? 0U : r.lane_mask; m != 0U; m &= m - 1U) {
+          words[__builtin_ctz(m)] += w;
+          tiles[__builtin_ctz(m)] += 1U;
+        }
+        if (r.lane_mask == d.valid_lane_mask) {
+          words[32] += w;
+          tiles[32] += 1U;
+        }
+      }
+      for (std::uint32_t l = 0; l < W; ++l) {
+        if ((d.valid_lane_mask >> l) & 1u) {
+          nets.push_back(bfx::ResidentNet{b, l, words[l] + words[32], tiles[l] + tiles[32]});
+        }
       }
       bfx::require(U > 0, "batch has no selected vertices");
       if (U > 0x7FFFFFFFull) throw std::overflow_error("union vertex count exceeds the device index range");
@@ -1566,7 +1613,7 @@ int bfx_prepare_batches(bfx_workspace* ws, uint32_t count, const bfx_batch_descr
         }
       }
     }
-    const bfx::Layout L = bfx::lay_out_batches(ws, count, sz);
+    const bfx::Layout L = bfx::lay_out_batches(ws, count, sz, nets);
     char* hb = static_cast<char*>(ws->staging.ptr);
     for (std::uint32_t b = 0; b < count; ++b) {
       const bfx_batch_description& d = batches[b];
@@ -1609,6 +1656,9 @@ int bfx_prepare_batches_from_queries(bfx_workspace* ws, uint32_t batch_count, co
     // indices, strictly increasing tiles and terminals in range.  Terminal
     // ownership is checked on the device.
     std::vector<std::uint8_t> used(query_count, 0);
+    std::vector<u32> query_words(query_count, 0U);  // 32-vertex words of a query's selected tiles
+    std::vector<bfx::ResidentNet> nets;
+    const auto& tvo = ws->graph->tile_vertex_offsets;
     std::vector<u32> lane_base(batch_count + 1, 0U), lane_query, lane_tile_base(1, 0U);
     std::vector<bfx::BatchSizes> sz(batch_count);
     for (u32 b = 0; b < batch_count; ++b) {
@@ -1629,6 +1679,7 @@ int bfx_prepare_batches_from_queries(bfx_workspace* ws, uint32_t batch_count, co
             if (r.selected_tiles[i] >= g.T) throw std::out_of_range("selected tile out of range");
             bfx::require(i == 0 || r.selected_tiles[i] > r.selected_tiles[i - 1],
                          "selected tiles must be strictly increasing");
+            query_words[qi] += (tvo[r.selected_tiles[i] + 1U] - tvo[r.selected_tiles[i]] + 31U) / 32U;
           }
           for (u32 i = 0; i < r.source_count; ++i) {
             if (r.sources[i] >= g.V) throw std::out_of_range("source out of range");
@@ -1642,6 +1693,7 @@ int bfx_prepare_batches_from_queries(bfx_workspace* ws, uint32_t batch_count, co
         }
         S += r.source_count;
         Tg += r.target_count;
+        nets.push_back(bfx::ResidentNet{b, l, query_words[qi], r.selected_tile_count});
         lane_query.push_back(qi);
         lane_tile_base.push_back(lane_tile_base.back() + r.selected_tile_count);
       }
@@ -1730,7 +1782,7 @@ int bfx_prepare_batches_from_queries(bfx_workspace* ws, uint32_t batch_count, co
       bfx::require(sz[b].U > 0, "batch has no selected vertices");
     }
     // Layout, records, then the description arrays written on the device.
-    const bfx::Layout L = bfx::lay_out_batches(ws, batch_count, sz);
+    const bfx::Layout L = bfx::lay_out_batches(ws, batch_count, sz, nets);
     bfx::upload(ws->meta.ptr, ws->staging.ptr, L.o_up, ws->stream);
     ws->last_h2d = image_bytes + L.o_up;
     u32* d_err = reinterpret_cast<u32*>(qb + o_err);
@@ -1932,6 +1984,24 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
     p.engines = upload_batch_words(ws, ws->engines_dev, ws->engines_uploaded, eng);
     p.engine = BFX_ENGINE_FRONTIER_PUSH;
   }
+  // Frontier lanes that fit a cluster's shared memory are relaxed there
+  // (resident.cu); what remains takes the grid-wide kernels.  Not for launches
+  // that may stop on their round limit (its labels carry no predecessors
+  // until they converge), that trace rounds, or that set a grid, a layout or
+  // an option of the grid-wide kernels.
+  const bool resident = ws->resident_mode != 0u && !ws->nets.empty() && p.flat == 2u &&
+                        ws->frontier_layout == BFX_FRONTIER_CHUNKED && p.engine == BFX_ENGINE_FRONTIER_PUSH &&
+                        o.maximum_rounds >= kResidentRounds && o.instrumentation < 2u && o.grid_policy == 0u &&
+                        ws->relax_atomic == 0u && ws->edge_major == 0u && ws->chunk_pairs == 0u &&
+                        ws->flat_items == 2u && ws->register_budget == 0u;
+  bool remaining = !resident;
+  if (resident) {
+    p.fit = ws->d_fit;
+    for (std::uint32_t b = 0; b < ws->nb && !remaining; ++b) {
+      const bool frontier = p.engines == nullptr || ws->engines_uploaded[b] == BFX_ENGINE_FRONTIER_PUSH;
+      remaining = !frontier || (ws->batches[b].valid & ~ws->fit[b]) != 0u;
+    }
+  }
   const int block = static_cast<int>(o.block_size);
   const size_t smem = (size_t{ws->nb} + 1) * 4;
   std::uint64_t launches = 0;
@@ -1971,9 +2041,11 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
     require(!(regs == 80u && p.flat == 2u && ws->chunk_pairs == 0u) || block <= 256,
             "the 80-register chunked kernel needs blocks of at most 256 threads");
     const int grid = grid_blocks(ws, kfn, block, smem, o);
-    void* args[] = {&p};
-    BFX_CUDA(cudaLaunchCooperativeKernel(kfn, grid, block, args, smem, ws->stream));
-    ++launches;
+    if (remaining) {
+      void* args[] = {&p};
+      BFX_CUDA(cudaLaunchCooperativeKernel(kfn, grid, block, args, smem, ws->stream));
+      ++launches;
+    }
   } else {
     const std::uint32_t K = o.control_mode == BFX_CONTROL_PER_ROUND_HOST_POLL ? 1u : o.rounds_per_chunk;
     const bool chunked = p.flat == 2u;
@@ -1990,7 +2062,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
     const bool reuse = ws->chunk_exec && ws->chunk_rounds == K && ws->chunk_grid == grid &&
                        ws->chunk_instr == o.instrumentation &&
                        ws->chunk_block == block && std::memcmp(&ws->chunk_params, &p, sizeof(p)) == 0;
-    if (!reuse) {
+    if (remaining && !reuse) {
       if (ws->chunk_exec) cudaGraphExecDestroy(ws->chunk_exec);
       ws->chunk_exec = nullptr;
       cudaGraph_t graph;
@@ -2042,6 +2114,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
       launches += 2ull * K;
     }
   }
+  if (resident) launches += launch_resident(ws, p, o.instrumentation != 0u);
   BFX_CUDA(cudaGetLastError());
   BFX_CUDA(cudaEventRecord(ws->ev[2], ws->stream));
   finalize_kernel<<<ws->nb, 256, 0, ws->stream>>>(p, ws->d_ctrl, ws->d_status);
@@ -2059,6 +2132,14 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
 }  // namespace bfx
 
 extern "C" {
+
+int bfx_set_resident_nets(bfx_workspace* ws, uint32_t mode) {
+  return bfx::guarded([&] {
+    bfx::require(ws != nullptr, "null argument");
+    bfx::require(mode <= 1u, "resident nets must be 0 or 1");
+    ws->resident_mode = mode;
+  });
+}
 
 int bfx_set_register_budget(bfx_workspace* ws, uint32_t registers) {
   return bfx::guarded([&] {

@@ -43,6 +43,7 @@ struct DGraph {
   const uint2* lrun;   // [V] own-tile run of each CSR row {first CSR index, count} (rows are sorted by
                        // destination tile, so a vertex's edges into its own tile are contiguous)
   const u32* tile_off; // [T+1] first vertex of each tile
+  const uint2* csr_row; // [V] {first CSR index, out-degree} (cluster-resident searches)
 };
 
 struct DBatch {
@@ -133,6 +134,10 @@ constexpr u32 kMaxBatchesPerLaunch = 4096;
 constexpr u64 kBarrierTimeoutNs = 2000000000ull;  // 2 s per barrier wait
 constexpr u64 kLaunchBudgetNs = 30000000000ull;   // 30 s per relaxation launch
 
+// Cluster-resident searches (resident.cu) need at least this round limit: a
+// launch that stops on its limit reports labels mid-way.
+constexpr u64 kResidentRounds = 65536u;
+
 struct LaunchParams {
   DGraph g;
   const DBatch* batches;
@@ -160,7 +165,14 @@ struct LaunchParams {
   u32 tile_wmax;         // tiled layout: widest batch of the launch (sizes the staged label rows)
   u32 tile_iters;        // tiled layout: local relaxation passes per visit before the rest waits a round
   u32 tshift;            // tiled layout: a dense round visits units of 2^tshift compact vertices (the tile size)
+  const u32* fit;        // [nb] lanes that the cluster-resident kernel relaxes (resident.cu), or null (none)
   const u32* mappings;   // tiled layout, [nb] or null (every batch visits tiles): BFX_MAPPING_* per batch
+};
+
+// One lane of a prepared batch: its selected tiles and the 32-vertex words
+// they fill when every tile starts on a word of its own.
+struct ResidentNet {
+  u32 batch, lane, words, tiles;
 };
 
 constexpr u32 kRoundTraceCap = 65536;
@@ -235,6 +247,11 @@ struct bfx_resident_graph {
   // the same power-of-two count of vertices in [32, 256], else 8 (units then
   // straddle tiles, which costs locality but not correctness); at least 5.
   std::uint32_t tile_shift{8};
+  // Cluster-resident searches: words (32 vertices, a tile starts on one) are
+  // dealt to blocks in runs of 2^word_run; word_whole: every tile is one run.
+  std::uint32_t word_run{3};
+  bool word_whole{false};
+  std::uint32_t resident_shapes{0};  // block configurations that the device holds
 };
 
 struct bfx_workspace {
@@ -281,6 +298,16 @@ struct bfx_workspace {
   std::uint64_t path_edges{0};
   bool paths_ready{false};
   bfx::DeviceBuffer adjoint;     // per-edge exact accumulators, upstream values, result
+  // Cluster-resident searches (resident.cu): the lanes that fit a cluster,
+  // largest first, and per batch the mask of those lanes; host and device.
+  std::vector<bfx::ResidentNet> nets;
+  std::vector<std::uint32_t> fit;
+  const bfx::ResidentNet* d_nets{nullptr};
+  const bfx::u32* d_fit{nullptr};
+  std::uint32_t resident_mode = 1;   // see bfx_set_resident_nets
+  cudaEvent_t resident_fork{nullptr};
+  std::vector<cudaStream_t> resident_streams;
+  std::vector<cudaEvent_t> resident_joins;
   std::vector<std::uint32_t> batch_engines;  // per-batch engine for BFX_ENGINE_AUTO launches
   std::vector<float> batch_deltas;           // per-batch near/far steps (empty: plain frontier)
   std::vector<std::uint32_t> batch_mappings; // tiled layout: per-batch dense-round mapping (empty: tile visits)

@@ -352,6 +352,15 @@ int bfx_set_batch_mappings(bfx_workspace *ws, uint32_t count, const uint32_t *ma
 /* The workspace's frontier layout and, for the first `count` batches, their
  * mappings (BFX_MAPPING_TILE_VISITS where none was set). */
 int bfx_get_frontier_mapping(bfx_workspace *ws, uint32_t *layout, uint32_t count, uint32_t *mappings);
+/* Cluster-resident searches (a bfx tuning option, results unchanged): with 1,
+ * the default, each frontier lane whose distances fit the shared memory of a
+ * thread-block cluster is relaxed by a cluster of its own, outside the
+ * grid-wide kernels; 0 relaxes every lane grid-wide.  Launches that set
+ * maximum_rounds below 65,536, an explicit grid, round tracing, another
+ * frontier layout or an option of the grid-wide kernels (bfx_set_register_budget,
+ * _flat_items, _flat_order, _relax_atomic, _chunk_pairs) stay grid-wide.  The
+ * round count of a batch is then the largest of its lanes'. */
+int bfx_set_resident_nets(bfx_workspace *ws, uint32_t mode);
 /* Register budget of the persistent relaxation kernel (a bfx tuning option,
  * results unchanged): 40 registers per thread (three 512-thread blocks per
  * SM), 64 (two 512-thread blocks per SM: no spills in the group layout, few
