@@ -196,43 +196,81 @@ __device__ void block_prefix(u32* prefix, u32 nb, F value, u32 kmax = 1u) {
 // Initialisation and seeding
 // ---------------------------------------------------------------------------
 
-// Grid-stride over all union vertices of all batches: compact->global map,
-// +inf labels, clear masks; over tile tables: {mask, bias} for union tiles.
+// Lanes of batch b that the grid-wide kernels relax (0: all lanes have
+// clusters of their own, and the batch needs labels only).
+__device__ __forceinline__ u32 grid_wide_lanes(const LaunchParams& p, u32 b) {
+  const u32 valid = p.batches[b].valid;
+  return p.fit != nullptr && engine_of(p, b) == BFX_ENGINE_FRONTIER_PUSH ? valid & ~p.fit[b] : valid;
+}
+
+// Calls body(b, first, last) for the union vertices [first, last) of batch b
+// that lie in a slice of kSlice union vertices, block by block; a portion's
+// labels are contiguous.
+constexpr u32 kSlice = 2048u;
+template <typename F>
+__device__ __forceinline__ void for_slices(const LaunchParams& p, F body) {
+  const u32 total = p.unit_base[p.nb];
+  for (u64 s = blockIdx.x; s * kSlice < total; s += gridDim.x) {
+    u32 u = static_cast<u32>(s) * kSlice;
+    const u32 end = min(total - u, kSlice) + u;
+    for (u32 b = find_batch(p.unit_base, p.nb, u); u < end; ++b) {
+      const u32 base = p.unit_base[b], last = min(end, p.unit_base[b + 1u]);
+      body(b, u - base, last - base);
+      u = last;
+    }
+  }
+}
+
+// Stores `word` to p[0 .. n), n of the block's threads together, 16 bytes a
+// thread where the start allows it.
+__device__ __forceinline__ void fill_words(u64* p, u64 n, u64 word) {
+  const u64 head = (reinterpret_cast<u64>(p) & 15u) != 0u && n != 0u ? 1u : 0u;
+  if (threadIdx.x < head) p[0] = word;
+  p += head;
+  n -= head;
+  const uint4 two = make_uint4(static_cast<u32>(word), dev::hi(word), static_cast<u32>(word), dev::hi(word));
+  for (u64 i = threadIdx.x; i < n / 2u; i += blockDim.x) reinterpret_cast<uint4*>(p)[i] = two;
+  if (threadIdx.x == 0u && (n & 1u) != 0u) p[n - 1u] = word;
+}
+
+// Labels of every union vertex of every batch (+inf, in whole rows: the init
+// writes as much as it can stream); for the batches that the grid-wide
+// kernels relax, the compact->global map, clear masks and the row tables; over
+// tile tables: {mask, bias} for union tiles.
 __global__ void init_kernel(LaunchParams p) {
   const u64 tid = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x;
   const u64 stride = static_cast<u64>(gridDim.x) * blockDim.x;
-  const u32 total_units = p.unit_base[p.nb];
-  for (u64 u = tid; u < total_units; u += stride) {
-    const u32 b = find_batch(p.unit_base, p.nb, static_cast<u32>(u));
+  for_slices(p, [&](u32 b, u32 first, u32 last) {
     const DBatch& B = p.batches[b];
-    const u32 cv = static_cast<u32>(u) - p.unit_base[b];
-    // range containing cv
-    u32 lo = 0, hi = B.range_count;
-    while (hi - lo > 1u) {
-      const u32 mid = (lo + hi) >> 1;
-      if (B.range_off[mid] <= cv) lo = mid; else hi = mid;
-    }
-    const uint4 r = B.ranges[lo];
-    B.c2g[cv] = r.y + (cv - B.range_off[lo]);
-    B.mask[0][cv] = 0u;
-    B.mask[1][cv] = 0u;
-    B.fmask[cv] = 0u;
-    B.fbound[cv] = 0xFFFFFFFFu;
-    if (p.flat >= 2u) {
-      if ((cv & 1023u) == 0u) {  // chunk bitmap words, one per 1,024 vertices (enough for any shift >= 5)
-        B.cmask[0][cv >> 10] = 0u;
-        B.cmask[1][cv >> 10] = 0u;
+    const u32 eng = engine_of(p, b), wide = grid_wide_lanes(p, b);
+    const u64 at = static_cast<u64>(first) << B.shift, n = static_cast<u64>(last - first) << B.shift;
+    fill_words(B.dist[0] + at, n, dev::kUnreached);
+    if (eng == BFX_ENGINE_JACOBI_PULL) fill_words(B.dist[1] + at, n, dev::kUnreached);
+    if (wide == 0u) return;
+    for (u32 cv = first + threadIdx.x; cv < last; cv += blockDim.x) {
+      // range containing cv
+      u32 lo = 0, hi = B.range_count;
+      while (hi - lo > 1u) {
+        const u32 mid = (lo + hi) >> 1;
+        if (B.range_off[mid] <= cv) lo = mid; else hi = mid;
       }
-      const u32 v = r.y + (cv - B.range_off[lo]);
-      const u32 rb = p.g.csr_off[v];
-      B.crow[cv] = make_uint2(rb, p.g.csr_off[v + 1u] - rb);
-      if (p.flat == 3u) B.clrun[cv] = p.g.lrun[v];
+      const u32 v = B.ranges[lo].y + (cv - B.range_off[lo]);
+      B.c2g[cv] = v;
+      B.mask[0][cv] = 0u;
+      B.mask[1][cv] = 0u;
+      B.fmask[cv] = 0u;
+      B.fbound[cv] = 0xFFFFFFFFu;
+      if (p.flat >= 2u) {
+        if ((cv & 1023u) == 0u) {  // chunk bitmap words, one per 1,024 vertices (enough for any shift >= 5)
+          B.cmask[0][cv >> 10] = 0u;
+          B.cmask[1][cv >> 10] = 0u;
+        }
+        const u32 rb = p.g.csr_off[v];
+        B.crow[cv] = make_uint2(rb, p.g.csr_off[v + 1u] - rb);
+        if (p.flat == 3u) B.clrun[cv] = p.g.lrun[v];
+      }
     }
-    for (u32 l = 0; l < B.W; ++l) {
-      B.dist[0][(static_cast<u64>(cv) << B.shift) + l] = dev::kUnreached;
-      if (engine_of(p, b) == BFX_ENGINE_JACOBI_PULL) B.dist[1][(static_cast<u64>(cv) << B.shift) + l] = dev::kUnreached;
-    }
-  }
+  });
   // Tile tables: clear every tile then write union tiles (a second pass in
   // the same kernel would race; clearing is done by the host-side memset).
   for (u32 b = 0; b < p.nb; ++b) {
@@ -287,13 +325,13 @@ __global__ void seed_kernel(LaunchParams p, const u32* src_base) {
       atomicOr(&p.ctl[b].error_bits, static_cast<u32>(BFX_DEVICE_ERROR_INVALID_CONTROLLER_STATE));
       continue;
     }
+    // a lane with a cluster of its own (resident.cu) finds its sources there
+    if (((grid_wide_lanes(p, b) >> lane) & 1u) == 0u) continue;
     const u32 cv = v - t.y;
-    B.dist[0][(static_cast<u64>(cv) << B.shift) + lane] = dev::kSourceWord;
     const u32 eng = engine_of(p, b);
+    B.dist[0][(static_cast<u64>(cv) << B.shift) + lane] = dev::kSourceWord;
     if (eng == BFX_ENGINE_JACOBI_PULL) B.dist[1][(static_cast<u64>(cv) << B.shift) + lane] = dev::kSourceWord;
-    if (eng == BFX_ENGINE_FRONTIER_PUSH && p.fit != nullptr && ((p.fit[b] >> lane) & 1u)) {
-      // relaxed by its own cluster (resident.cu), which finds its sources itself
-    } else if (eng == BFX_ENGINE_FRONTIER_PUSH && p.flat >= 2u) {
+    if (eng == BFX_ENGINE_FRONTIER_PUSH && p.flat >= 2u) {
       // chunked / tiled frontier: pending lane, then the claim unit's bit;
       // the thread that sets the bit queues the unit
       atomicOr(&B.mask[0][cv], 1u << lane);
@@ -870,29 +908,22 @@ __global__ void expand_lane_kernel(DGraph g, DBatch B, u32 slot, u32 lane, u32* 
   }
 }
 
-// Largest finite distance bits per batch over the final labels (grid-stride
-// over the union vertices of all batches, as init_kernel); out[b] starts at 0.
+// Largest finite distance bits per batch over the final labels, read in order;
+// out[b] starts at 0.
 __global__ void label_bound_kernel(LaunchParams p, const bfx_device_run_status* statuses, u32* out) {
-  const u64 tid = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const u64 stride = static_cast<u64>(gridDim.x) * blockDim.x;
-  const u32 total_units = p.unit_base[p.nb];
-  u32 best = 0u, best_b = 0xFFFFFFFFu;
-  for (u64 u = tid; u < total_units; u += stride) {
-    const u32 b = find_batch(p.unit_base, p.nb, static_cast<u32>(u));
-    if (b != best_b) {
-      if (best_b != 0xFFFFFFFFu && best != 0u) atomicMax(out + best_b, best);
-      best_b = b;
-      best = 0u;
-    }
+  for_slices(p, [&](u32 b, u32 first, u32 last) {
     const DBatch& B = p.batches[b];
-    const u32 cv = static_cast<u32>(u) - p.unit_base[b];
-    const u64* const d = B.dist[statuses[b].final_distance_slot] + (static_cast<u64>(cv) << B.shift);
-    for (u32 l = 0; l < B.W; ++l) {
-      const u32 h = dev::hi(d[l]);
-      if (h < dev::kInfBits && h > best) best = h;
+    const u64* const d = B.dist[statuses[b].final_distance_slot] + (static_cast<u64>(first) << B.shift);
+    const u64 n = static_cast<u64>(last - first) << B.shift;
+    u32 best = 0u;
+#pragma unroll 4
+    for (u64 i = threadIdx.x; i < n; i += blockDim.x) {
+      const u32 h = dev::hi(d[i]);
+      if (h < dev::kInfBits) best = max(best, h);
     }
-  }
-  if (best_b != 0xFFFFFFFFu && best != 0u) atomicMax(out + best_b, best);
+    best = __reduce_max_sync(0xFFFFFFFFu, best);
+    if (lane_id() == 0u && best != 0u) atomicMax(out + b, best);
+  });
 }
 
 // ---------------------------------------------------------------------------

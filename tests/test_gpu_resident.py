@@ -71,7 +71,8 @@ def test_tile_sizes(gpu, nodes, step):
 @pytest.mark.parametrize("side", [4, 20, 45, 64, 80, 110, 124, 160])
 def test_net_sizes(gpu, side):
     """One net per launch: side^2 x 32 vertices take one block to the largest
-    clusters; the largest does not fit and stays grid-wide."""
+    clusters; the two largest (with their tables of one-word tiles) do not fit
+    and stay grid-wide."""
     layout, grid = graph("c1", 160, 160, 32)
     queries = workloads.box_queries(layout, grid, 1, side, side, seed=side, targets=(3, 3))
     descs = bfx.make_overlapping_batch_plan(layout, queries, POLICY).descriptions()
