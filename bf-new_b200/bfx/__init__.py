@@ -638,8 +638,8 @@ class Workspace:
         _check(load().bfx_set_register_budget(self._h, u32(registers)))
 
     def set_resident_nets(self, mode: int):
-        """1 (default): frontier lanes that fit a thread-block cluster's shared memory are relaxed there;
-        0: every lane takes the grid-wide kernels."""
+        """1 (default): frontier lanes that fit a thread-block cluster's shared memory are relaxed there, larger
+        whole-graph lanes by a team of blocks each; 0: every lane takes the grid-wide kernels."""
         _check(load().bfx_set_resident_nets(self._h, u32(mode)))
 
     def set_chunk_pairs(self, mode: int):

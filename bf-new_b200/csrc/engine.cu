@@ -244,7 +244,8 @@ __global__ void init_kernel(LaunchParams p) {
     const DBatch& B = p.batches[b];
     const u32 eng = engine_of(p, b), wide = grid_wide_lanes(p, b);
     const u64 at = static_cast<u64>(first) << B.shift, n = static_cast<u64>(last - first) << B.shift;
-    fill_words(B.dist[0] + at, n, dev::kUnreached);
+    // (a team's batch gets its label rows whole)
+    if (wide != 0u || B.team == 0u) fill_words(B.dist[0] + at, n, dev::kUnreached);
     if (eng == BFX_ENGINE_JACOBI_PULL) fill_words(B.dist[1] + at, n, dev::kUnreached);
     if (wide == 0u) return;
     for (u32 cv = first + threadIdx.x; cv < last; cv += blockDim.x) {
@@ -1399,8 +1400,10 @@ struct Layout {
 Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector<BatchSizes>& sz,
                        std::vector<ResidentNet>& nets) {
   const DGraph& g = ws->graph->g;
-  std::vector<u32> fit(count, 0u);
-  resident_select(ws, nets, fit);
+  std::vector<u32> fit(count, 0u), full(count);
+  for (std::uint32_t b = 0; b < count; ++b) full[b] = sz[b].full;
+  std::vector<ResidentNet> whole;
+  resident_select(ws, full, nets, whole, fit);
   const size_t o_batch = 0;
   const size_t o_ctl = align256(o_batch + count * sizeof(DBatch));
   const size_t o_run = align256(o_ctl + count * sizeof(DCtl));
@@ -1411,7 +1414,9 @@ Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector
   const size_t o_fit = align256(o_ctrl + count * sizeof(bfx_device_controller));
   const size_t o_nets = align256(o_fit + count * 4);
   Layout L;
-  L.o_up = align256(o_nets + nets.size() * sizeof(ResidentNet));
+  const size_t o_whole = align256(o_nets + nets.size() * sizeof(ResidentNet));
+  const size_t o_teams = align256(o_whole + whole.size() * sizeof(ResidentNet));
+  L.o_up = align256(o_teams + kMaxTeams * sizeof(TeamState));
   L.arrays.resize(count);
   size_t up = L.o_up;
   for (std::uint32_t b = 0; b < count; ++b) {
@@ -1515,7 +1520,12 @@ Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector
   }
   ubase[count] = static_cast<std::uint32_t>(usum);
   sbase[count] = static_cast<std::uint32_t>(ssum);
+  for (const ResidentNet& n : whole) ws->batches[n.batch].team = 1u;
   std::memcpy(hb + o_batch, ws->batches.data(), count * sizeof(DBatch));
+  if (!whole.empty()) std::memcpy(hb + o_whole, whole.data(), whole.size() * sizeof(ResidentNet));
+  ws->whole.swap(whole);
+  ws->d_whole = reinterpret_cast<const ResidentNet*>(db + o_whole);
+  ws->d_teams = reinterpret_cast<TeamState*>(db + o_teams);
   std::memcpy(hb + o_fit, fit.data(), count * 4);
   if (!nets.empty()) std::memcpy(hb + o_nets, nets.data(), nets.size() * sizeof(ResidentNet));
   ws->fit.swap(fit);
@@ -2020,9 +2030,9 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
   // that may stop on their round limit (its labels carry no predecessors
   // until they converge), that trace rounds, or that set a grid, a layout or
   // an option of the grid-wide kernels.
-  const bool resident = ws->resident_mode != 0u && !ws->nets.empty() && p.flat == 2u &&
+  const bool resident = ws->resident_mode != 0u && !(ws->nets.empty() && ws->whole.empty()) && p.flat == 2u &&
                         ws->frontier_layout == BFX_FRONTIER_CHUNKED && p.engine == BFX_ENGINE_FRONTIER_PUSH &&
-                        o.maximum_rounds >= kResidentRounds && o.instrumentation < 2u && o.grid_policy == 0u &&
+                        o.maximum_rounds >= kLateRounds && o.instrumentation < 2u && o.grid_policy == 0u &&
                         ws->relax_atomic == 0u && ws->edge_major == 0u && ws->chunk_pairs == 0u &&
                         ws->flat_items == 2u && ws->register_budget == 0u;
   bool remaining = !resident;
@@ -2145,7 +2155,10 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
       launches += 2ull * K;
     }
   }
-  if (resident) launches += launch_resident(ws, p, o.instrumentation != 0u);
+  if (resident) {
+    launches += launch_teams(ws, p, o.instrumentation != 0u);
+    launches += launch_resident(ws, p, o.instrumentation != 0u);
+  }
   BFX_CUDA(cudaGetLastError());
   BFX_CUDA(cudaEventRecord(ws->ev[2], ws->stream));
   finalize_kernel<<<ws->nb, 256, 0, ws->stream>>>(p, ws->d_ctrl, ws->d_status);

@@ -49,6 +49,7 @@ struct DGraph {
 struct DBatch {
   u32 W, shift, valid, U;
   u32 src_count, tgt_count, range_count;
+  u32 team;            // whole-graph batch whose lanes teams of blocks relax where LaunchParams::fit is set
   u32 full;            // every tile selected by every valid lane, compact index == vertex id
   u64* dist[2];        // [U*W] labels (slot 1 only for Jacobi)
   u32* mask[2];        // [U] pending lane masks (frontier)
@@ -134,9 +135,10 @@ constexpr u32 kMaxBatchesPerLaunch = 4096;
 constexpr u64 kBarrierTimeoutNs = 2000000000ull;  // 2 s per barrier wait
 constexpr u64 kLaunchBudgetNs = 30000000000ull;   // 30 s per relaxation launch
 
-// Cluster-resident searches (resident.cu) need at least this round limit: a
-// launch that stops on its limit reports labels mid-way.
-constexpr u64 kResidentRounds = 65536u;
+// Searches that find predecessors after convergence (resident.cu) need at
+// least this round limit: a launch that stops on its
+// limit reports labels mid-way.
+constexpr u64 kLateRounds = 65536u;
 
 struct LaunchParams {
   DGraph g;
@@ -165,7 +167,7 @@ struct LaunchParams {
   u32 tile_wmax;         // tiled layout: widest batch of the launch (sizes the staged label rows)
   u32 tile_iters;        // tiled layout: local relaxation passes per visit before the rest waits a round
   u32 tshift;            // tiled layout: a dense round visits units of 2^tshift compact vertices (the tile size)
-  const u32* fit;        // [nb] lanes that the cluster-resident kernel relaxes (resident.cu), or null (none)
+  const u32* fit;        // [nb] lanes that clusters or teams of blocks relax (resident.cu), or null (none)
   const u32* mappings;   // tiled layout, [nb] or null (every batch visits tiles): BFX_MAPPING_* per batch
 };
 
@@ -174,6 +176,16 @@ struct LaunchParams {
 struct ResidentNet {
   u32 batch, lane, words, tiles;
 };
+
+// Barrier and rotating flags of a team of blocks (resident.cu).
+struct TeamState {
+  dev::GridSync sync;
+  u32 any[3];    // a vertex is pending: by round % 3
+  u32 moved[3];  // a split moved a vertex: by split % 3
+  u32 least[3];  // complement of the smallest far distance, by split % 3
+  u32 reserved[51];
+};
+constexpr u32 kMaxTeams = 8u;
 
 constexpr u32 kRoundTraceCap = 65536;
 
@@ -300,9 +312,11 @@ struct bfx_workspace {
   bfx::DeviceBuffer adjoint;     // per-edge exact accumulators, upstream values, result
   // Cluster-resident searches (resident.cu): the lanes that fit a cluster,
   // largest first, and per batch the mask of those lanes; host and device.
-  std::vector<bfx::ResidentNet> nets;
+  std::vector<bfx::ResidentNet> nets, whole;  // whole: whole-graph lanes that no cluster holds
   std::vector<std::uint32_t> fit;
   const bfx::ResidentNet* d_nets{nullptr};
+  const bfx::ResidentNet* d_whole{nullptr};
+  bfx::TeamState* d_teams{nullptr};
   const bfx::u32* d_fit{nullptr};
   std::uint32_t resident_mode = 1;   // see bfx_set_resident_nets
   cudaEvent_t resident_fork{nullptr};

@@ -1,6 +1,6 @@
-// Cluster-resident frontier searches: one lane (net) of a batch is relaxed by
-// one thread-block cluster whose shared memories hold all of the net's
-// distances.
+// Frontier searches outside the grid-wide kernels: one lane (net) of a batch is
+// relaxed by one thread-block cluster whose shared memories hold all of the
+// net's distances; larger whole-graph lanes by a team of blocks (below).
 //
 // What bounds the grid-wide frontier (frontier.cuh) on regional sets is the
 // memory system: every relaxation reads a random 8-byte label, the labels of
@@ -64,6 +64,7 @@ constexpr u32 kShapeCount = sizeof(kShapes) / sizeof(kShapes[0]);
 // at least 64 words (2,048 vertices) a block: below that a round is its fixed
 // latency (one 4,096-vertex net: 0.10 ms on 4 blocks, 0.23 ms on one).
 constexpr size_t kLaunchStreams = 4;
+constexpr u64 kTeamBytes = u64{270} << 20;
 constexpr u32 kSpreadShape = 7u, kSpreadWords = 64u;
 
 __host__ __device__ __forceinline__ u32 block_words(u32 words, u32 ctas, u32 run) {
@@ -659,6 +660,402 @@ __global__ void __launch_bounds__(1024, 1)
   cluster_sync(ctas);  // neighbours may still read this block's distances
 }
 
+// ---------------------------------------------------------------------------
+// Whole-graph lanes: a team of blocks per lane, distances in global memory.
+//
+// A lane over the whole graph needs no tile table (compact index = vertex) but
+// no cluster holds it.  Its 32-bit distances and bitmaps are 4.4 bytes a
+// vertex, so with a few lanes in progress most random reads of a relaxation
+// stay in the L2 (the grid-wide frontier relaxes all lanes of a batch at once,
+// and its label rows of 8 bytes a lane come from DRAM).  The rounds are the
+// cluster searches', with a barrier over the team's blocks.  The label rows
+// are written and the predecessors found for all lanes of a batch together.
+// B200, relaxation launches before and after: 32 lanes of 4.2M vertices 63.0
+// -> 22.8 ms (20.1 of it the searches, 110 G edges/s, 2.6 TB/s of DRAM; 2.5
+// the predecessors), 64 lanes of 16.8M vertices 567 -> 205 ms, one lane of
+// 2.1M vertices 4.1 -> 2.9 ms.
+// ---------------------------------------------------------------------------
+
+// Scratch of a lane, in the batch's second label slot (8 bytes a vertex and
+// lane): distances, two pending bitmaps, the far bitmap.
+struct LaneScratch {
+  u32 *L, *near0, *near1, *far;
+};
+__device__ __forceinline__ LaneScratch lane_scratch(const DBatch& B, u32 V, u32 ql) {
+  LaneScratch s;
+  s.L = reinterpret_cast<u32*>(B.dist[1] + static_cast<u64>(V) * ql);
+  s.near0 = s.L + V;
+  s.near1 = s.near0 + ((V + 31u) >> 5);
+  s.far = s.near1 + ((V + 31u) >> 5);
+  return s;
+}
+
+constexpr u32 kTeamList = 4096u;  // pending vertices of a block's pass
+
+template <bool kCount>
+__global__ void __launch_bounds__(1024, 1)
+    team_kernel(LaunchParams p, const ResidentNet* nets, u32 net_count, u32 teams, TeamState* states) {
+  __shared__ u32 s_list[kTeamList];
+  __shared__ u32 s_listed[2], s_cut[2], s_min[32];
+  const u32 per = gridDim.x / teams, team = blockIdx.x / per, rank = blockIdx.x - team * per;
+  if (team >= teams) return;
+  TeamState& S = states[team];
+  const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, warps = blockDim.x >> 5;
+  const u32 V = p.g.V, words = (V + 31u) >> 5;
+  const u64 t0 = dev::global_ns();
+  if (tid < 2u) {
+    s_listed[tid] = 0u;
+    s_cut[tid] = kFull;
+  }
+  u32 r = 0u, splits = 0u, pass = 0u;  // rounds and splits of the team so far: its flags rotate over them
+  u64 cnt[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  const auto barrier = [&]() {
+    if (dev::grid_barrier(&S.sync, per, kBarrierTimeoutNs)) return true;
+    if (tid == 0u) atomicExch(&p.run->abort, 1u);
+    return false;
+  };
+  for (u32 n = team; n < net_count; n += teams) {
+    const u32 b = nets[n].batch, ql = nets[n].lane;
+    if (engine_of(p, b) != BFX_ENGINE_FRONTIER_PUSH) continue;
+    const DBatch& B = p.batches[b];
+    DCtl& C = p.ctl[b];
+    const LaneScratch m = lane_scratch(B, V, ql);
+    const u64 at = static_cast<u64>(rank) * blockDim.x + tid, stride = static_cast<u64>(per) * blockDim.x;
+    for (u64 i = at; i < V; i += stride) m.L[i] = dev::kInfBits;
+    for (u64 i = at; i < 3ull * words; i += stride) m.near0[i] = 0u;
+    if (!barrier()) return;
+    if (rank == 0u) {
+      for (u32 i = B.src_off[ql] + tid; i < B.src_off[ql + 1u]; i += blockDim.x) {
+        const u32 v = B.src[i];
+        m.L[v] = 0u;
+        dev::red_or(m.near0 + (v >> 5), 1u << (v & 31u));
+      }
+    }
+    if (!barrier()) return;
+    const u32 delta = p.deltas ? p.deltas[b] : dev::kInfBits;
+    u32 tau = delta, rounds = 0u;
+    for (;; ++rounds) {
+      u32* const cur = (rounds & 1u) ? m.near1 : m.near0;
+      u32* const nxt = (rounds & 1u) ? m.near0 : m.near1;
+      bool any = false;
+      const auto relax = [&](u32 v, uint2 row, u32 take) {
+        u32 d = dev::kInfBits;
+        if (lane < take) {
+          d = dev::ld_cg(m.L + v);
+          if (kCount) {
+            cnt[0] += 1u;
+            cnt[1] += row.y;
+            cnt[2] += 1u;
+            cnt[3] += row.y;
+          }
+        }
+        const EdgeList edges(row, take);
+        for (u32 base = 0; base < edges.total; base += 32u * kSteps) {
+          uint2 rec[kSteps];
+          u32 cand[kSteps], x[kSteps];
+#pragma unroll
+          for (u32 k = 0; k < kSteps; ++k) {
+            u32 from;
+            bool live;
+            const u32 e = edges.edge(base + k * 32u, from, live);
+            rec[k] = make_uint2(0u, kFull);  // NaN weight: improves nothing
+            if (live) rec[k] = __ldg(reinterpret_cast<const uint2*>(p.g.csr + e));
+            cand[k] = __shfl_sync(kFull, d, static_cast<int>(from));
+          }
+#pragma unroll
+          for (u32 k = 0; k < kSteps; ++k) {
+            cand[k] = __float_as_uint(__fadd_rn(__uint_as_float(cand[k]), __uint_as_float(rec[k].y)));
+            x[k] = rec[k].y != kFull ? dev::ld_cg(m.L + rec[k].x) : 0u;
+          }
+#pragma unroll
+          for (u32 k = 0; k < kSteps; ++k) {
+            if (cand[k] < x[k]) {
+              dev::red_min_u32(m.L + rec[k].x, cand[k]);
+              const bool near = cand[k] < tau;
+              any |= near;
+              dev::red_or((near ? nxt : m.far) + (rec[k].x >> 5), 1u << (rec[k].x & 31u));
+              if (kCount) {
+                cnt[5] += 1u;
+                cnt[6] += 1u;
+              }
+            }
+          }
+        }
+      };
+      // The block's words: groups of 32 dealt over the team's blocks.
+      for (;; ++pass) {
+        for (u32 g = rank + warp * per; g * 32u < words; g += warps * per) {
+          const u32 w = g * 32u + lane;
+          u32 bits = w < words ? dev::ld_cg(cur + w) : 0u;
+          const u32 c = static_cast<u32>(__popc(bits));
+          u32 to = c;
+          for (u32 o = 1; o < 32u; o <<= 1) {
+            const u32 y = __shfl_up_sync(kFull, to, o);
+            if (lane >= o) to += y;
+          }
+          const u32 total = __shfl_sync(kFull, to, 31);
+          if (total == 0u) continue;
+          u32 first = 0u;
+          if (lane == 31u) {
+            first = atomicAdd(&s_listed[pass & 1u], total);
+            if (first + total > kTeamList) atomicMin(&s_cut[pass & 1u], first);
+          }
+          first = __shfl_sync(kFull, first, 31);
+          if (first + total > kTeamList) continue;  // the words keep their bits for the next pass
+          to += first - c;
+          if (bits != 0u) cur[w] = 0u;
+          for (; bits != 0u; bits &= bits - 1u) s_list[to++] = w * 32u + static_cast<u32>(__ffs(bits)) - 1u;
+        }
+        __syncthreads();
+        const u32 cut = s_cut[pass & 1u], listed = min(s_listed[pass & 1u], cut);
+        if (tid == 0u) {  // the next pass's; its readers of the pass before passed the barrier above
+          s_listed[(pass + 1u) & 1u] = 0u;
+          s_cut[(pass + 1u) & 1u] = kFull;
+        }
+        const u32 share = listed > 16u * warps ? 32u : (listed > 8u * warps ? 16u : 8u);
+        u32 i = warp * share, v = 0u;
+        uint2 row = make_uint2(0u, 0u);
+        const auto fetch = [&](u32 from) {
+          row = make_uint2(0u, 0u);
+          if (lane < share && from + lane < listed) {
+            v = s_list[from + lane];
+            row = __ldg(p.g.csr_row + v);
+          }
+        };
+        if (i < listed) fetch(i);
+        for (; i < listed; i += warps * share) {
+          const u32 this_v = v;
+          const uint2 this_row = row;
+          if (i + warps * share < listed) fetch(i + warps * share);
+          relax(this_v, this_row, min(share, listed - i));
+        }
+        if (cut == kFull) break;
+        __syncthreads();
+      }
+      ++pass;
+      if (__syncthreads_or(any) && tid == 0u) atomicExch(&S.any[r % 3u], 1u);
+      if ((r & 63u) == 63u && rank == 0u && tid == 0u && dev::global_ns() - t0 > p.budget_ns) {
+        atomicExch(&S.sync.abort, 1u);
+      }
+      if (!barrier()) return;
+      const bool more = dev::ld_cg(&S.any[r % 3u]) != 0u;
+      // the slot of the round after next; its last readers passed the barrier above
+      if (rank == 0u && tid == 0u) S.any[(r + 2u) % 3u] = 0u;
+      ++r;
+      if (more) continue;
+
+      // --- split: far vertices below the next threshold become pending ---------
+      // The first scan takes tau + delta; where that moves none, the second
+      // takes the smallest far distance + delta.
+      bool converged = false;
+      const u32 old = tau;
+      for (u32 scan = 0;; ++scan) {
+        if (scan == 0u) tau = __float_as_uint(__fadd_rn(__uint_as_float(tau), __uint_as_float(delta)));
+        u32 least = dev::kInfBits;
+        bool moved = false;
+        for (u32 g = rank + warp * per; g * 32u < words; g += warps * per) {
+          const u32 w = g * 32u + lane;
+          const u32 f = w < words ? dev::ld_cg(m.far + w) : 0u;
+          u32 keep = f, move = 0u;
+          // eight words at a time, a word's 32 distances one read
+          for (u32 todo = __ballot_sync(kFull, f != 0u); todo != 0u;) {
+            u32 from[8], x[8];
+#pragma unroll
+            for (u32 k = 0; k < 8u; ++k) {
+              from[k] = todo != 0u ? static_cast<u32>(__ffs(todo)) - 1u : 32u;
+              todo &= todo - 1u;
+            }
+#pragma unroll
+            for (u32 k = 0; k < 8u; ++k) {
+              const u32 y = from[k] < 32u ? (g * 32u + from[k]) * 32u + lane : V;
+              x[k] = y < V ? dev::ld_cg(m.L + y) : dev::kInfBits;
+            }
+#pragma unroll
+            for (u32 k = 0; k < 8u; ++k) {
+              if (from[k] == 32u) continue;  // warp-uniform
+              const bool mine = ((__shfl_sync(kFull, f, static_cast<int>(from[k])) >> lane) & 1u) != 0u;
+              // below the old threshold: was pending when it got there
+              const u32 stay = __ballot_sync(kFull, mine && x[k] >= tau);
+              const u32 go = __ballot_sync(kFull, mine && x[k] < tau && x[k] >= old);
+              if (mine && x[k] >= tau) least = min(least, x[k]);
+              if (lane == from[k]) {
+                keep = stay;
+                move = go;
+              }
+            }
+          }
+          if (keep != f) m.far[w] = keep;
+          if (move != 0u) {
+            nxt[w] = move;  // empty before the split
+            moved = true;
+          }
+        }
+        least = __reduce_min_sync(kFull, least);
+        if (lane == 0u) s_min[warp] = least;
+        const bool block_moved = __syncthreads_or(moved) != 0;
+        if (warp == 0u) {
+          least = __reduce_min_sync(kFull, lane < warps ? s_min[lane] : dev::kInfBits);
+          if (lane == 0u) {
+            atomicMax(&S.least[splits % 3u], ~least);
+            if (block_moved) atomicExch(&S.moved[splits % 3u], 1u);
+          }
+        }
+        if (!barrier()) return;
+        least = ~dev::ld_cg(&S.least[splits % 3u]);
+        const bool go = dev::ld_cg(&S.moved[splits % 3u]) != 0u;
+        if (rank == 0u && tid == 0u) S.least[(splits + 2u) % 3u] = S.moved[(splits + 2u) % 3u] = 0u;
+        ++splits;
+        if (go) break;
+        if (least >= dev::kInfBits) {
+          converged = true;
+          break;
+        }
+        const u32 stepped = __float_as_uint(__fadd_rn(__uint_as_float(least), __uint_as_float(delta)));
+        tau = max(stepped, least + 1u);
+      }
+      if (converged) break;
+    }
+    if (tid == 0u && rank == 0u) {
+      atomicMax(&C.rounds, rounds + 1u);
+      atomicMax(reinterpret_cast<unsigned long long*>(&p.run->work[7]), static_cast<unsigned long long>(rounds + 1u));
+    }
+  }
+  if (kCount) {
+    for (int i = 0; i < 7; ++i) {
+      u64 x = cnt[i];
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(kFull, x, o);
+      if (lane == 0u && x) atomicAdd(reinterpret_cast<unsigned long long*>(&p.run->work[i]), x);
+    }
+  }
+}
+
+// Label rows of a whole-graph batch from its lanes' distances, the predecessor
+// word unreached: a warp turns 32 vertices x W lanes through shared memory.
+__global__ void __launch_bounds__(256) team_rows_kernel(LaunchParams p, u32 b) {
+  __shared__ u32 s_rows[8][32 * 33];
+  if (engine_of(p, b) != BFX_ENGINE_FRONTIER_PUSH) return;
+  const DBatch& B = p.batches[b];
+  const u32 V = p.g.V, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  u32* const rows = s_rows[warp];
+  for (u32 v0 = (blockIdx.x * 8u + warp) * 32u; v0 < V; v0 += gridDim.x * 256u) {
+    for (u32 l = 0; l < B.W; ++l) {
+      u32 x = dev::kInfBits;
+      if (((B.valid >> l) & 1u) && v0 + lane < V) x = lane_scratch(B, V, l).L[v0 + lane];
+      rows[lane * 33u + l] = x;
+    }
+    __syncwarp();
+    const u32 n = min(V - v0, 32u) << B.shift;
+    u64* const out = B.dist[0] + (static_cast<u64>(v0) << B.shift);
+    for (u32 k = lane; k < n; k += 32u) {
+      out[k] = (static_cast<u64>(rows[(k >> B.shift) * 33u + (k & (B.W - 1u))]) << 32) | kFull;
+    }
+    __syncwarp();
+  }
+}
+
+// Predecessors of a whole-graph batch, in place (distances are the high words,
+// which no thread writes): per (vertex, lane) the smallest stable edge id
+// among the in-edges that give its distance.
+__global__ void __launch_bounds__(256) team_predecessor_kernel(LaunchParams p, u32 b) {
+  __shared__ u32 s_best[8][32];
+  if (engine_of(p, b) != BFX_ENGINE_FRONTIER_PUSH) return;
+  const DBatch& B = p.batches[b];
+  const u32 V = p.g.V, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const auto source = [&](u32 v, u32 ql) {
+    u32 lo = B.src_off[ql], hi = B.src_off[ql + 1u];
+    const u32 end = hi;
+    while (lo < hi) {
+      const u32 mid = (lo + hi) >> 1;
+      if (B.src[mid] < v) lo = mid + 1u; else hi = mid;
+    }
+    return lo < end && B.src[lo] == v;
+  };
+  u32* const words = reinterpret_cast<u32*>(B.dist[0]);  // {predecessor, distance} pairs
+  if (B.W == 1u) {
+    // 32 vertices' in-edges as one list
+    volatile u32* const best = s_best[warp];
+    for (u32 v0 = (blockIdx.x * 8u + warp) * 32u; v0 < V; v0 += gridDim.x * 256u) {
+      const u32 v = v0 + lane;
+      const u32 d = v < V ? words[2ull * v + 1u] : dev::kInfBits;
+      uint2 col = make_uint2(0u, 0u);
+      if (d < dev::kInfBits) {
+        col.x = __ldg(p.g.csc_off + v);
+        col.y = __ldg(p.g.csc_off + v + 1u) - col.x;
+      }
+      best[lane] = kFull;
+      __syncwarp();
+      const EdgeList edges(col, 32u);
+      for (u32 base = 0; base < edges.total; base += 32u * kSteps) {
+        uint4 rec[kSteps];
+        u32 from[kSteps], x[kSteps];
+#pragma unroll
+        for (u32 k = 0; k < kSteps; ++k) {
+          bool live;
+          const u32 e = edges.edge(base + k * 32u, from[k], live);
+          rec[k] = make_uint4(0u, kFull, kFull, 0u);
+          if (live) rec[k] = __ldg(p.g.csc + e);
+        }
+#pragma unroll
+        for (u32 k = 0; k < kSteps; ++k) x[k] = rec[k].y != kFull ? words[2ull * rec[k].x + 1u] : dev::kInfBits;
+#pragma unroll
+        for (u32 k = 0; k < kSteps; ++k) {
+          const u32 dv = __shfl_sync(kFull, d, static_cast<int>(from[k]));
+          if (__float_as_uint(__fadd_rn(__uint_as_float(x[k]), __uint_as_float(rec[k].y))) == dv) {
+            shared_min<false>(shared_address(const_cast<u32*>(best + from[k])), rec[k].z, true);
+          }
+        }
+      }
+      __syncwarp();
+      if (d < dev::kInfBits) words[2ull * v] = d == 0u && source(v, 0u) ? 0u : best[lane];
+      __syncwarp();
+    }
+    return;
+  }
+  // W threads per vertex, one per lane; they read its in-edge records together
+  // and then each its own distances, four in-edges in flight.
+  const u32 W = B.W, ql = lane & (W - 1u), vpw = 32u >> B.shift;
+  for (u32 v0 = (blockIdx.x * 8u + warp) * vpw; v0 < V; v0 += gridDim.x * 8u * vpw) {
+    const u32 v = v0 + (lane >> B.shift);
+    const u64 at = (static_cast<u64>(v) << B.shift) + ql;
+    u32 d = dev::kInfBits, cb = 0u, count = 0u;
+    if (v < V) {
+      d = words[2u * at + 1u];
+      cb = __ldg(p.g.csc_off + v);
+      count = __ldg(p.g.csc_off + v + 1u) - cb;
+    }
+    u32 eid = kFull;
+    const u32 most = __reduce_max_sync(kFull, count);
+    for (u32 e = 0; e < most; e += W) {
+      uint4 mine = make_uint4(0u, kFull, kFull, 0u);  // NaN weight: gives no distance
+      if (e + ql < count) mine = __ldg(p.g.csc + cb + e + ql);
+      const u32 here = min(W, most - e);
+      for (u32 k = 0; k < here; k += 4u) {
+        u32 u[4], w[4], id[4], x[4];
+#pragma unroll
+        for (u32 j = 0; j < 4u; ++j) {
+          const int from = static_cast<int>(min(k + j, W - 1u));
+          u[j] = __shfl_sync(kFull, mine.x, from, static_cast<int>(W));
+          w[j] = __shfl_sync(kFull, mine.y, from, static_cast<int>(W));
+          id[j] = __shfl_sync(kFull, mine.z, from, static_cast<int>(W));
+        }
+#pragma unroll
+        for (u32 j = 0; j < 4u; ++j) {
+          x[j] = w[j] != kFull ? words[2u * ((static_cast<u64>(u[j]) << B.shift) + ql) + 1u] : dev::kInfBits;
+        }
+#pragma unroll
+        for (u32 j = 0; j < 4u; ++j) {
+          if (__float_as_uint(__fadd_rn(__uint_as_float(x[j]), __uint_as_float(w[j]))) == d) eid = min(eid, id[j]);
+        }
+      }
+    }
+    if (d < dev::kInfBits) words[2u * at] = d == 0u && source(v, ql) ? 0u : eid;
+  }
+}
+
+const void* team_entry(bool count) {
+  return count ? reinterpret_cast<const void*>(team_kernel<true>) : reinterpret_cast<const void*>(team_kernel<false>);
+}
+
 const void* resident_entry(bool count, bool cluster, bool whole) {
   if (!cluster) {  // one block: a tile is contiguous in any case
     return count ? reinterpret_cast<const void*>(resident_kernel<true, false, true>)
@@ -732,7 +1129,8 @@ u32 resident_shapes() {
   return shapes;
 }
 
-void resident_select(bfx_workspace* ws, std::vector<ResidentNet>& nets, std::vector<u32>& fit) {
+void resident_select(bfx_workspace* ws, const std::vector<u32>& full, std::vector<ResidentNet>& nets,
+                     std::vector<ResidentNet>& whole, std::vector<u32>& fit) {
   const bfx_resident_graph* graph = ws->graph;
   const u32 run = graph->word_run, shapes = graph->resident_shapes;
   std::sort(nets.begin(), nets.end(), [](const ResidentNet& a, const ResidentNet& b) {
@@ -740,16 +1138,61 @@ void resident_select(bfx_workspace* ws, std::vector<ResidentNet>& nets, std::vec
   });
   std::vector<ResidentNet> kept;
   kept.reserve(nets.size());
+  whole.clear();
   for (const ResidentNet& n : nets) {
-    if (smallest_shape(graph, n, run, shapes) == kShapeCount) continue;
-    kept.push_back(n);
+    if (smallest_shape(graph, n, run, shapes) != kShapeCount) {
+      kept.push_back(n);
+    } else if (full[n.batch] != 0u) {
+      whole.push_back(n);
+    } else {
+      continue;
+    }
     fit[n.batch] |= 1u << n.lane;
   }
   nets.swap(kept);
+  // lanes of a batch in turn, batch by batch
+  std::sort(whole.begin(), whole.end(), [](const ResidentNet& a, const ResidentNet& b) {
+    return a.batch != b.batch ? a.batch < b.batch : a.lane < b.lane;
+  });
+}
+
+u32 launch_teams(bfx_workspace* ws, const LaunchParams& p, bool count) {
+  if (ws->whole.empty()) return 0;
+  // Lanes at a time: as many as kTeamBytes of distances allow, in equal turns.
+  // More teams hide one another's barriers and read latency, until their wave
+  // fronts outgrow the L2.  Measured (ms): 32 lanes of 4.2M vertices (17 MB)
+  // on 1 / 2 / 4 / 8 / 16 teams 51.5 / 33.8 / 25.9 / 22.8 / 22.4; 64 lanes of
+  // 16.8M vertices (67 MB) on 1 / 2 / 4 / 6 / 8 / 16 teams 297 / 227 / 205 /
+  // 231 / 223 / 259.
+  u32 lanes = static_cast<u32>(ws->whole.size());
+  const u64 lane_bytes = static_cast<u64>(p.g.V) * 4u;
+  const u32 most = std::max(1u, std::min(kMaxTeams, static_cast<u32>(kTeamBytes / lane_bytes)));
+  u32 teams = (lanes + most - 1u) / most;  // turns
+  teams = (lanes + teams - 1u) / teams;
+  const ResidentNet* d_whole = ws->d_whole;
+  TeamState* states = ws->d_teams;
+  BFX_CUDA(cudaMemsetAsync(states, 0, sizeof(TeamState) * kMaxTeams, ws->stream));
+  LaunchParams params = p;
+  void* args[] = {&params, &d_whole, &lanes, &teams, &states};
+  BFX_CUDA(cudaLaunchCooperativeKernel(team_entry(count), dim3(static_cast<u32>(ws->sm_count) / teams * teams),
+                                       dim3(1024), args, 0, ws->stream));
+  u32 launches = 1;
+  for (u32 i = 0, last = 0xFFFFFFFFu; i < lanes; ++i) {
+    const u32 b = ws->whole[i].batch;
+    if (b == last) continue;
+    last = b;
+    team_rows_kernel<<<ws->sm_count * 6, 256, 0, ws->stream>>>(params, b);
+    BFX_CUDA(cudaGetLastError());
+    team_predecessor_kernel<<<ws->sm_count * 8, 256, 0, ws->stream>>>(params, b);
+    BFX_CUDA(cudaGetLastError());
+    launches += 2;
+  }
+  return launches;
 }
 
 u32 launch_resident(bfx_workspace* ws, const LaunchParams& p, bool count) {
   const std::vector<ResidentNet>& nets = ws->nets;
+  if (nets.empty()) return 0;
   const u32 run = ws->graph->word_run;
   const u32 shapes = ws->graph->resident_shapes;
   // A net takes the smallest shape that holds it; where the nets together

@@ -9,9 +9,15 @@ namespace bfx {
 // smallest); called once per resident graph.
 u32 resident_shapes();
 
-// Sorts the prepared set's lanes largest first, drops those that no cluster
-// holds, and sets fit[b] to the lanes of batch b that stay.
-void resident_select(bfx_workspace* ws, std::vector<ResidentNet>& nets, std::vector<u32>& fit);
+// Sorts the prepared set's lanes largest first and keeps in `nets` those that
+// a cluster holds; larger lanes of whole-graph batches (full[b]) go to `whole`
+// (a team of blocks each); fit[b] gets the lanes of batch b in either.
+void resident_select(bfx_workspace* ws, const std::vector<u32>& full, std::vector<ResidentNet>& nets,
+                     std::vector<ResidentNet>& whole, std::vector<u32>& fit);
+
+// Launches the whole-graph lanes' searches on ws->stream; returns the number
+// of launches.
+u32 launch_teams(bfx_workspace* ws, const LaunchParams& p, bool count);
 
 // Launches the searches of the prepared set's nets (those of batches on
 // another engine return at once).  The work is ordered after what ws->stream

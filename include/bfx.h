@@ -354,8 +354,9 @@ int bfx_set_batch_mappings(bfx_workspace *ws, uint32_t count, const uint32_t *ma
 int bfx_get_frontier_mapping(bfx_workspace *ws, uint32_t *layout, uint32_t count, uint32_t *mappings);
 /* Cluster-resident searches (a bfx tuning option, results unchanged): with 1,
  * the default, each frontier lane whose distances fit the shared memory of a
- * thread-block cluster is relaxed by a cluster of its own, outside the
- * grid-wide kernels; 0 relaxes every lane grid-wide.  Launches that set
+ * thread-block cluster is relaxed by a cluster of its own, and each larger
+ * whole-graph lane by a team of thread blocks, outside the grid-wide kernels;
+ * 0 relaxes every lane grid-wide.  Launches that set
  * maximum_rounds below 65,536, an explicit grid, round tracing, another
  * frontier layout or an option of the grid-wide kernels (bfx_set_register_budget,
  * _flat_items, _flat_order, _relax_atomic, _chunk_pairs) stay grid-wide.  The

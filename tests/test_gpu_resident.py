@@ -1,5 +1,6 @@
-"""Cluster-resident searches (bfx_set_resident_nets): the lanes that fit a
-thread-block cluster's shared memory are relaxed there.  Their labels must be
+"""Searches outside the grid-wide kernels (bfx_set_resident_nets): the lanes
+that fit a thread-block cluster's shared memory are relaxed there, larger
+whole-graph lanes by a team of blocks each.  Their labels must be
 the oracle's and the grid-wide kernels', bit for bit, for tiles of one word,
 whole runs of words and ragged sizes, for nets from one block to clusters of
 16, beside lanes that stay grid-wide in the same launch, and in every control
@@ -79,6 +80,40 @@ def test_net_sizes(gpu, side):
     here, wide = compare(layout, queries, descs, 40.0, lanes=1)
     # init, seed, one relaxation launch, finalize, either way
     assert here == wide == 4
+
+
+@pytest.mark.parametrize("step", [None, 3.0, 200.0])
+@pytest.mark.parametrize("lanes,nodes", [(1, 45), (7, 64), (12, 45), (20, 33)])
+def test_whole_graph_lanes(gpu, lanes, nodes, step):
+    """Whole-graph lanes that no cluster holds, one team of blocks each: lane
+    widths 1, 8, 16 and 32, fewer lanes than teams and more, vertex counts that
+    are and are not a multiple of a word, weights of zero."""
+    layout, grid = graph("c1f", 151, 157, nodes)
+    rng = np.random.default_rng(lanes)
+    resident = bfx.ResidentDeviceGraph.upload_once(layout)
+    a = layout.arrays
+    weights = np.zeros(layout.edge_count, np.float32)
+    weights[a["csr_edge_ids"]] = a["csr_weights"]
+    weights[rng.integers(0, layout.edge_count, 2000)] = 0.0
+    resident.set_weights(weights)
+    a["csr_weights"] = weights[a["csr_edge_ids"]]
+    a["csc_weights"] = weights[a["csc_edge_ids"]]
+    queries = workloads.full_graph_queries(layout, grid, lanes, 9, targets_per_query=5)
+    descs = bfx.make_overlapping_batch_plan(layout, queries, bfx.BatchPlannerPolicy(32, 0, 1, 10000, 1,
+                                                                                   narrow_lanes=True)).descriptions()
+    wide = relax(resident, descs, 0, step)
+    for options in ({}, {"instrumentation": 1}):
+        here = relax(resident, descs, 1, step, **options)
+        assert here[0] == wide[0] and all(s["stop_reason"] == bfx.STOP_CONVERGED for s in here[0])
+        for x, y in zip(here[1], wide[1]):
+            np.testing.assert_array_equal(x[0], y[0])
+            np.testing.assert_array_equal(x[1], y[1])
+    resident.close()
+    orc = Oracle.from_layout(layout)
+    q = queries[int(descs[0].query_index_by_lane[0])]
+    dist, pred = orc.region_sssp(q.sources, q.targets, q.selected_tiles)
+    np.testing.assert_array_equal(here[1][0][0][:, 0], dist)
+    np.testing.assert_array_equal(here[1][0][1][:, 0], pred)
 
 
 @pytest.mark.parametrize("control", [bfx.CONTROL_PERSISTENT, bfx.CONTROL_CHUNKED, bfx.CONTROL_PER_ROUND])
