@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -39,7 +40,7 @@ struct DGraph {
   const uint4* csr;    // [E] {dst, weight bits, eid+1, dst tile}
   const u32* csc_off;  // [V+1]
   const uint4* csc;    // [E] {src, weight bits, eid+1, src tile}
-  const u32* eid_src;  // [E] source vertex of each stable edge id
+  const uint2* eid_src; // [E] source vertex of each stable edge id and that vertex's tile
   const uint2* lrun;   // [V] own-tile run of each CSR row {first CSR index, count} (rows are sorted by
                        // destination tile, so a vertex's edges into its own tile are contiguous)
   const u32* tile_off; // [T+1] first vertex of each tile
@@ -278,6 +279,8 @@ struct bfx_workspace {
   bfx::DeviceBuffer arena;  // labels, masks, queues, c2g, row tables
   bfx::DeviceBuffer tile_tables;  // per batch dense {lane mask, compact bias} over all tiles
   bfx::DeviceBuffer qimage;       // device-side preparation: the uploaded query and lane image
+  bfx::DeviceBuffer image;        // label images and path payloads on their way to the host
+  bfx::PinnedBuffer image_host;
   bfx::PinnedBuffer staging;
   bfx::PinnedBuffer status_host;
   size_t meta_bytes{0};
@@ -341,3 +344,16 @@ struct bfx_workspace {
   bfx::DeviceBuffer round_trace;  // instrumentation 2 only
 };
 
+namespace bfx {
+
+// Device bytes of a download at a time, at most.
+constexpr size_t kImageBytes = size_t{64} << 20;
+
+struct HostImage {
+  const void* device;
+  void* host;
+  size_t bytes;
+};
+void fetch_images(bfx_workspace* ws, std::initializer_list<HostImage> images);
+
+}  // namespace bfx

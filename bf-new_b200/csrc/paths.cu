@@ -18,7 +18,12 @@
 //
 // Two passes as in the reference: summaries (status, source, distance,
 // length), then, after a host prefix over the lengths, the payload (path
-// vertices source-first, their labels, stable edge ids).
+// vertices source-first, their labels, stable edge ids).  The walk is a chain
+// of dependent reads (edge -> source and its tile -> tile entry -> label,
+// about 2 us a step on a B200), so it is walked once: the summaries pass
+// keeps each target's edges (a trail), and the payload and the adjoint take a
+// trail with a warp, all its edges at once.  Paths longer than a trail are
+// walked again.
 #include "bfx.h"
 #include "bfx_internal.hpp"
 #include "device_common.cuh"
@@ -58,6 +63,8 @@ struct PathArgs {
   u32 slots;
   u64 slot_stride;
   u64 mark_stride;
+  u32* trail;          // [targets * trail_cap] a target's path edges, target first
+  u32 trail_cap;
   u32* flagged;        // [targets] indices of the targets the walk handed over
   u32* flagged_count;  // [1]
 };
@@ -84,6 +91,15 @@ __device__ __forceinline__ u64 label(const DGraph& g, const DBatch& B, const u64
   const uint2 t = B.tiles[g.owner[v]];
   if (((t.x >> lane) & 1u) == 0u) return dev::kUnreached;
   return d[(static_cast<u64>(v - t.y) << B.shift) + lane];
+}
+
+// The label of the source of edge e, and that source.
+__device__ __forceinline__ u64 source_label(const DGraph& g, const DBatch& B, const u64* d, u32 e, u32 lane, u32& u) {
+  const uint2 src = g.eid_src[e];
+  u = src.x;
+  const uint2 t = B.full ? make_uint2(B.valid, 0u) : B.tiles[src.y];
+  if (((t.x >> lane) & 1u) == 0u) return dev::kUnreached;
+  return d[(static_cast<u64>(u - t.y) << B.shift) + lane];
 }
 
 __device__ __forceinline__ bool clean(const bfx_device_run_status& s) {
@@ -127,8 +143,8 @@ __global__ void summaries_kernel(PathArgs a) {
             fallback = true;
             break;
           }
-          const u32 u = a.g.eid_src[e];
-          const u64 wu = label(a.g, B, d, u, lane);
+          u32 u;
+          const u64 wu = source_label(a.g, B, d, e, lane, u);
           if (dev::hi(wu) == dev::kInfBits) {  // inconsistent chain: let the search decide
             fallback = true;
             break;
@@ -144,6 +160,7 @@ __global__ void summaries_kernel(PathArgs a) {
           } else {
             pn = 0u;
           }
+          if (len < a.trail_cap) a.trail[static_cast<u64>(i) * a.trail_cap + len] = e;
           ++len;
           if (len > B.U) {
             fallback = true;
@@ -287,10 +304,13 @@ __global__ void search_kernel(PathArgs a, bool payload) {
   }
 }
 
-// Pass 2: one thread per complete, walkable target writes its payload.
+// Pass 2: one warp per complete, walkable target writes its payload from the
+// target's trail, one edge per thread; a path longer than its trail is walked
+// by one thread.
 __global__ void payload_kernel(PathArgs a) {
-  const u32 total = a.target_base[a.batch_count];
-  for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+  const u32 total = a.target_base[a.batch_count], thread = threadIdx.x & 31u;
+  const u32 warps = (gridDim.x * blockDim.x) >> 5;
+  for (u32 i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < total; i += warps) {
     const u32 len = a.lengths[i];
     if ((len & kFallback) != 0u || a.summaries[i].reconstruction != 0u) continue;
     const u32 bi = find_b(a.target_base, a.batch_count, i);
@@ -300,6 +320,23 @@ __global__ void payload_kernel(PathArgs a) {
     const u32 lane = lane_of(B.tgt_off, B.W, pos);
     const u64* d = B.dist[a.status[b].final_distance_slot];
     const u64 vo = a.vertex_offsets[i], eo = a.edge_offsets[i];
+    if (len <= a.trail_cap) {
+      if (thread == 0u) {
+        const u32 t = B.tgt[pos];
+        a.out_vertices[vo + len] = t;
+        a.out_labels[vo + len] = __uint_as_float(dev::hi(label(a.g, B, d, t, lane)));
+      }
+      for (u32 k = thread; k < len; k += 32u) {
+        const u32 e = a.trail[static_cast<u64>(i) * a.trail_cap + k];
+        u32 u;
+        const u64 w = source_label(a.g, B, d, e, lane, u);
+        a.out_edges[eo + len - 1u - k] = e;
+        a.out_vertices[vo + len - 1u - k] = u;
+        a.out_labels[vo + len - 1u - k] = __uint_as_float(dev::hi(w));
+      }
+      continue;
+    }
+    if (thread != 0u) continue;
     u32 v = B.tgt[pos];
     u64 w = label(a.g, B, d, v, lane);
     for (u32 k = 0;; ++k) {
@@ -308,8 +345,7 @@ __global__ void payload_kernel(PathArgs a) {
       if (k == len) break;
       const u32 e = static_cast<u32>(w) - 1u;
       a.out_edges[eo + len - 1u - k] = e;
-      v = a.g.eid_src[e];
-      w = label(a.g, B, d, v, lane);
+      w = source_label(a.g, B, d, e, lane, v);
     }
   }
 }
@@ -397,12 +433,22 @@ __device__ float exact_round(const unsigned long long* acc) {
   return neg ? -r : r;
 }
 
+// One warp per target over its trail; a path longer than its trail is walked.
 __global__ void adjoint_walk_kernel(PathArgs a, const float* grads, unsigned long long* acc) {
-  const u32 total = a.target_base[a.batch_count];
-  for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    if ((a.lengths[i] & kFallback) != 0u || a.summaries[i].reconstruction != 0u) continue;
+  const u32 total = a.target_base[a.batch_count], thread = threadIdx.x & 31u;
+  const u32 warps = (gridDim.x * blockDim.x) >> 5;
+  for (u32 i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < total; i += warps) {
+    const u32 len = a.lengths[i];
+    if ((len & kFallback) != 0u || a.summaries[i].reconstruction != 0u) continue;
     const float g = grads[i];
     if (g == 0.0f) continue;
+    if (len <= a.trail_cap) {
+      for (u32 k = thread; k < len; k += 32u) {
+        exact_add(acc + 4ull * a.trail[static_cast<u64>(i) * a.trail_cap + k], g);
+      }
+      continue;
+    }
+    if (thread != 0u) continue;
     const u32 bi = find_b(a.target_base, a.batch_count, i);
     const u32 b = a.first_batch + bi;
     const DBatch& B = a.batches[b];
@@ -413,7 +459,8 @@ __global__ void adjoint_walk_kernel(PathArgs a, const float* grads, unsigned lon
     while (static_cast<u32>(w) != 0u) {
       const u32 e = static_cast<u32>(w) - 1u;
       exact_add(acc + 4ull * e, g);
-      w = label(a.g, B, d, a.g.eid_src[e], lane);
+      u32 u;
+      w = source_label(a.g, B, d, e, lane, u);
     }
   }
 }
@@ -452,12 +499,14 @@ void check_ready(bfx_workspace* ws) {
 
 // Layout of the workspace's path buffer for `targets` targets of
 // `batch_count` batches whose largest union has `max_union` vertices:
-// target prefix, summaries, walk lengths, payload offsets, the flagged list,
-// then the search slots (stacks and on-path bitmaps).  The number of slots is
-// what fits a 256 MB scratch budget (at least 1, at most 256).
+// target prefix, summaries, walk lengths, payload offsets, trails, the flagged
+// list, then the search slots (stacks and on-path bitmaps).  The number of
+// slots is what fits a 256 MB scratch budget (at least 1, at most 256), the
+// edges of a trail what fits 64 MB (at most 128: the paths of the regional
+// and full-graph configurations have up to 61).
 struct PathLayout {
-  size_t o_tb, o_sum, o_len, o_vo, o_eo, o_fl, o_fc, o_sv, o_sc, o_se, o_op, total;
-  u32 slots;
+  size_t o_tb, o_sum, o_len, o_vo, o_eo, o_tr, o_fl, o_fc, o_sv, o_sc, o_se, o_op, total;
+  u32 slots, trail_cap;
   u64 slot_stride, mark_stride;
 };
 
@@ -472,7 +521,9 @@ PathLayout path_layout(std::uint64_t T, std::uint32_t batch_count, std::uint32_t
   L.o_len = align256(L.o_sum + T * sizeof(bfx_compact_target_summary));
   L.o_vo = align256(L.o_len + T * 4);
   L.o_eo = align256(L.o_vo + T * 8);
-  L.o_fl = align256(L.o_eo + T * 8);
+  L.trail_cap = static_cast<u32>(std::min<size_t>(128, (size_t{64} << 20) / 4 / std::max<size_t>(1, T)));
+  L.o_tr = align256(L.o_eo + T * 8);
+  L.o_fl = align256(L.o_tr + T * L.trail_cap * 4);
   L.o_fc = align256(L.o_fl + T * 4);
   L.o_sv = align256(L.o_fc + 4);
   L.o_sc = L.o_sv + size_t{L.slots} * L.slot_stride * 4;
@@ -496,6 +547,8 @@ PathArgs path_args_at(bfx_workspace* ws, const PathLayout& L, std::uint32_t firs
   a.lengths = reinterpret_cast<std::uint32_t*>(base + L.o_len);
   a.vertex_offsets = reinterpret_cast<const std::uint64_t*>(base + L.o_vo);
   a.edge_offsets = reinterpret_cast<const std::uint64_t*>(base + L.o_eo);
+  a.trail = reinterpret_cast<std::uint32_t*>(base + L.o_tr);
+  a.trail_cap = L.trail_cap;
   a.flagged = reinterpret_cast<std::uint32_t*>(base + L.o_fl);
   a.flagged_count = reinterpret_cast<std::uint32_t*>(base + L.o_fc);
   a.stack_v = reinterpret_cast<std::uint32_t*>(base + L.o_sv);
@@ -549,21 +602,26 @@ int bfx_compact_path_summaries(bfx_workspace* ws, uint32_t first_batch, uint32_t
     BFX_CUDA(cudaMemsetAsync(base + L.o_fc, 0, 4, ws->stream));
     const bfx::PathArgs a = bfx::path_args_at(ws, L, first_batch, batch_count, max_union);
     if (T > 0) {
-      const int blocks = static_cast<int>(std::min<std::uint64_t>((T + 255) / 256, 4096));
-      bfx::summaries_kernel<<<blocks, 256, 0, ws->stream>>>(a);
+      // (32-thread blocks: the walks are latency, so they spread over the SMs)
+      const int walkers = static_cast<int>(std::min<std::uint64_t>((T + 31) / 32, 16384));
+      bfx::summaries_kernel<<<walkers, 32, 0, ws->stream>>>(a);
       BFX_CUDA(cudaGetLastError());
+      const int blocks = static_cast<int>(std::min<std::uint64_t>((T + 255) / 256, 4096));
       bfx::flag_list_kernel<<<blocks, 256, 0, ws->stream>>>(a);
       BFX_CUDA(cudaGetLastError());
       bfx::search_kernel<<<(a.slots + 31) / 32, 32, 0, ws->stream>>>(a, false);
       BFX_CUDA(cudaGetLastError());
     }
-    ws->paths_host.reserve(T * sizeof(bfx_compact_target_summary) + 256);
+    const size_t h_vo = bfx::align256(T * sizeof(bfx_compact_target_summary));
+    if (h_vo + T * 16 + 256 > ws->paths_host.bytes) BFX_CUDA(cudaStreamSynchronize(ws->stream));  // still read
+    ws->paths_host.reserve(h_vo + T * 16 + 256);
     BFX_CUDA(cudaMemcpyAsync(ws->paths_host.ptr, a.summaries, T * sizeof(bfx_compact_target_summary),
                              cudaMemcpyDeviceToHost, ws->stream));
     BFX_CUDA(cudaStreamSynchronize(ws->stream));
     std::memcpy(summaries, ws->paths_host.ptr, T * sizeof(bfx_compact_target_summary));
     // Payload offsets (checked host prefix, as the reference does).
-    std::vector<std::uint64_t> vo(T), eo(T);
+    auto* const vo = reinterpret_cast<std::uint64_t*>(static_cast<char*>(ws->paths_host.ptr) + h_vo);
+    auto* const eo = vo + T;
     std::uint64_t nv = 0, ne = 0;
     for (std::uint64_t i = 0; i < T; ++i) {
       vo[i] = nv;
@@ -573,9 +631,10 @@ int bfx_compact_path_summaries(bfx_workspace* ws, uint32_t first_batch, uint32_t
         ne += summaries[i].path_length;
       }
     }
-    BFX_CUDA(cudaMemcpyAsync(base + L.o_vo, vo.data(), T * 8, cudaMemcpyHostToDevice, ws->stream));
-    BFX_CUDA(cudaMemcpyAsync(base + L.o_eo, eo.data(), T * 8, cudaMemcpyHostToDevice, ws->stream));
-    BFX_CUDA(cudaStreamSynchronize(ws->stream));
+    // (pinned and not waited for: a later call waits for the stream before it
+    // writes them again)
+    BFX_CUDA(cudaMemcpyAsync(base + L.o_vo, vo, T * 8, cudaMemcpyHostToDevice, ws->stream));
+    BFX_CUDA(cudaMemcpyAsync(base + L.o_eo, eo, T * 8, cudaMemcpyHostToDevice, ws->stream));
     ws->path_first_batch = first_batch;
     ws->path_batch_count = batch_count;
     ws->path_targets = T;
@@ -597,32 +656,23 @@ int bfx_compact_path_payload(bfx_workspace* ws, uint32_t* vertices, float* dista
     bfx::require(vertices && distance_labels && (edge_ids || ws->path_edges == 0), "null output");
     BFX_CUDA(cudaSetDevice(ws->graph->device));
     const std::uint64_t T = ws->path_targets, nv = ws->path_vertices, ne = ws->path_edges;
-    // Output arena: vertices, labels, edges in one device allocation.
+    // Output arena: vertices, labels, edges, kept in the workspace.
     const size_t out_bytes = bfx::align256(nv * 4) * 2 + bfx::align256(ne * 4 + 4);
-    char* dout = nullptr;
-    BFX_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&dout), out_bytes, ws->stream));
+    ws->image.reserve(out_bytes, ws->graph->device);
+    char* const dout = static_cast<char*>(ws->image.ptr);
     bfx::PathArgs a = bfx::path_args(ws);
     a.out_vertices = reinterpret_cast<std::uint32_t*>(dout);
     a.out_labels = reinterpret_cast<float*>(dout + bfx::align256(nv * 4));
     a.out_edges = reinterpret_cast<std::uint32_t*>(dout + 2 * bfx::align256(nv * 4));
-    cudaError_t err = cudaSuccess;
     if (T > 0) {
-      const int blocks = static_cast<int>(std::min<std::uint64_t>((T + 255) / 256, 4096));
+      const int blocks = static_cast<int>(std::min<std::uint64_t>((T + 7) / 8, 4096));
       bfx::payload_kernel<<<blocks, 256, 0, ws->stream>>>(a);
-      err = cudaGetLastError();
-      if (err == cudaSuccess) {
-        bfx::search_kernel<<<(a.slots + 31) / 32, 32, 0, ws->stream>>>(a, true);
-        err = cudaGetLastError();
-      }
+      BFX_CUDA(cudaGetLastError());
+      bfx::search_kernel<<<(a.slots + 31) / 32, 32, 0, ws->stream>>>(a, true);
+      BFX_CUDA(cudaGetLastError());
     }
-    if (err == cudaSuccess && nv) {
-      cudaMemcpyAsync(vertices, a.out_vertices, nv * 4, cudaMemcpyDeviceToHost, ws->stream);
-      cudaMemcpyAsync(distance_labels, a.out_labels, nv * 4, cudaMemcpyDeviceToHost, ws->stream);
-    }
-    if (err == cudaSuccess && ne) cudaMemcpyAsync(edge_ids, a.out_edges, ne * 4, cudaMemcpyDeviceToHost, ws->stream);
-    cudaFreeAsync(dout, ws->stream);
-    BFX_CUDA(err);
-    BFX_CUDA(cudaStreamSynchronize(ws->stream));
+    bfx::fetch_images(ws, {{a.out_vertices, vertices, nv * 4}, {a.out_labels, distance_labels, nv * 4},
+                           {a.out_edges, edge_ids, ne * 4}});
   });
 }
 
@@ -655,7 +705,7 @@ extern "C" int bfx_edge_usage_adjoint(bfx_workspace* ws, const float* target_gra
     if (T) BFX_CUDA(cudaMemcpyAsync(g, target_grads, T * 4, cudaMemcpyHostToDevice, ws->stream));
     const bfx::PathArgs a = bfx::path_args(ws);
     if (T) {
-      const int blocks = static_cast<int>(std::min<std::uint64_t>((T + 255) / 256, 4096));
+      const int blocks = static_cast<int>(std::min<std::uint64_t>((T + 7) / 8, 4096));
       bfx::adjoint_walk_kernel<<<blocks, 256, 0, ws->stream>>>(a, g, acc);
       BFX_CUDA(cudaGetLastError());
       bfx::adjoint_search_kernel<<<(a.slots + 31) / 32, 32, 0, ws->stream>>>(a, g, acc);
