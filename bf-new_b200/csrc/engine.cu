@@ -1274,6 +1274,7 @@ int bfx_resident_graph_upload(const bfx_device_graph_layout32* layout, int devic
     double wsum = 0.0;
     for (std::uint32_t e = 0; e < E; ++e) wsum += L.csr_weights[e];
     G->mean_weight = E ? wsum / E : 0.0;
+    G->current_mean = G->mean_weight;
     G->g.V = V;
     G->g.E = E;
     G->g.T = T;
@@ -2057,6 +2058,9 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
   p.budget_ns = kLaunchBudgetNs;
   p.engines = nullptr;
   p.deltas = nullptr;
+  const float auto_step = kAutoSteps * static_cast<float>(ws->graph->current_mean);
+  std::memcpy(&p.auto_step, &auto_step, 4);
+  if (!(auto_step > 0.0f)) p.auto_step = dev::kInfBits;  // no edges, or none with a weight: plain
   p.flat = ws->frontier_layout == BFX_FRONTIER_FLAT ? 1u : (ws->frontier_layout == BFX_FRONTIER_CHUNKED ? 2u : 0u);
   p.cshift = 5u;
   p.cpack = ws->chunk_pack;

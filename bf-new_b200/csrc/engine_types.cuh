@@ -141,6 +141,12 @@ constexpr u64 kLaunchBudgetNs = 30000000000ull;   // 30 s per relaxation launch
 // limit reports labels mid-way.
 constexpr u64 kLateRounds = 65536u;
 
+// Near/far step of a set that was given none, in mean edge weights.  Plain
+// frontiers (one round per hop) relax 2.5 to 3 times as many edges as steps of
+// 4 on the regional and whole-graph configurations; steps of 2 to 8 are within
+// a tenth of one another.
+constexpr float kAutoSteps = 4.0f;
+
 struct LaunchParams {
   DGraph g;
   const DBatch* batches;
@@ -156,6 +162,8 @@ struct LaunchParams {
   u64 budget_ns;         // wall-clock budget of one relaxation launch; past it the launch stops (device_failure)
   const u32* engines;    // [nb] per-batch engine (autotuned launches) or null
   const u32* deltas;     // [nb] near/far threshold steps (float bits) or null (plain frontier)
+  u32 auto_step;         // step of the searches of resident.cu where `deltas` is null (float bits): kAutoSteps
+                         // mean edge weights
   u64* round_trace;      // instrumentation 2: per round {start %globaltimer, warp items | split batches << 32,
                          // active pairs, lane-edge relaxations}; null otherwise
   u32 trace_cap;         // rounds the trace holds
@@ -255,7 +263,8 @@ struct bfx_resident_graph {
   bfx::DeviceBuffer mem;
   std::vector<std::uint32_t> tile_vertex_offsets;  // host copy, [T+1]
   std::uint64_t bytes{0};
-  double mean_weight{0.0};
+  double mean_weight{0.0};   // of the uploaded weights (the tuner's set classes)
+  double current_mean{0.0};  // of the weights set last
   // Tiled frontier claim unit: log2 of the tile size when every tile holds
   // the same power-of-two count of vertices in [32, 256], else 8 (units then
   // straddle tiles, which costs locality but not correctness); at least 5.

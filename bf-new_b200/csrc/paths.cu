@@ -740,6 +740,8 @@ extern "C" int bfx_resident_graph_set_weights(bfx_resident_graph* graph, const f
       if (!(x >= 0.0f) || x == __builtin_inff()) throw std::invalid_argument("edge weights must be finite and nonnegative");
       if (x == 0.0f) x = 0.0f;  // canonical +0 (InputGraph canonicalisation)
     }
+    double sum = 0.0;
+    for (const float x : w) sum += x;
     BFX_CUDA(cudaSetDevice(graph->device));
     float* d = nullptr;
     BFX_CUDA(cudaMalloc(reinterpret_cast<void**>(&d), size_t{E} * 4 + 4));
@@ -752,5 +754,6 @@ extern "C" int bfx_resident_graph_set_weights(bfx_resident_graph* graph, const f
     }
     cudaFree(d);
     BFX_CUDA(err);
+    graph->current_mean = E ? sum / E : 0.0;
   });
 }

@@ -143,6 +143,13 @@ __device__ __forceinline__ void cluster_sync(u32 ctas) {
   }
 }
 
+// The step of a set without steps of its own (LaunchParams::auto_step) after
+// its n-th split: doubled every eighth time, so that weights which spread over
+// many orders of magnitude cost a logarithm of splits and not one per band.
+__device__ __forceinline__ u32 grown_step(u32 step, u32 n) {
+  return (n & 7u) == 0u ? __float_as_uint(__fadd_rn(__uint_as_float(step), __uint_as_float(step))) : step;
+}
+
 struct NetShared {
   u32 scan[33];
   u32 any[3];                  // a vertex is pending: by round % 3
@@ -373,7 +380,7 @@ __global__ void __launch_bounds__(1024, 1)
   cluster_sync(ctas);
 
   // --- rounds ------------------------------------------------------------------
-  const u32 delta = p.deltas ? p.deltas[b] : dev::kInfBits;
+  u32 delta = p.deltas ? p.deltas[b] : p.auto_step;
   u32 tau = delta, splits = 0u, rounds = 0u, pass = 0u;
   u32 cnt[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
   u64 total_cnt[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
@@ -558,6 +565,7 @@ __global__ void __launch_bounds__(1024, 1)
     for (u32 i = 0; i < ctas; ++i) least = min(least, s.fmin[splits & 1u][i]);
     if (least >= dev::kInfBits) break;  // nothing far: converged
     ++splits;
+    if (p.deltas == nullptr) delta = grown_step(delta, splits);
     const u32 stepped = __float_as_uint(__fadd_rn(__uint_as_float(least), __uint_as_float(delta)));
     tau = max(stepped, least + 1u);  // at least the next float above the smallest far distance
     for (u32 w = tid; w < M; w += blockDim.x) {
@@ -732,8 +740,9 @@ __global__ void __launch_bounds__(1024, 1)
       }
     }
     if (!barrier()) return;
-    const u32 delta = p.deltas ? p.deltas[b] : dev::kInfBits;
+    u32 delta = p.deltas ? p.deltas[b] : p.auto_step;
     u32 tau = delta, rounds = 0u;
+    const u32 splits0 = splits;
     for (;; ++rounds) {
       u32* const cur = (rounds & 1u) ? m.near1 : m.near0;
       u32* const nxt = (rounds & 1u) ? m.near0 : m.near1;
@@ -905,6 +914,7 @@ __global__ void __launch_bounds__(1024, 1)
         const bool go = dev::ld_cg(&S.moved[splits % 3u]) != 0u;
         if (rank == 0u && tid == 0u) S.least[(splits + 2u) % 3u] = S.moved[(splits + 2u) % 3u] = 0u;
         ++splits;
+        if (p.deltas == nullptr) delta = grown_step(delta, splits - splits0);
         if (go) break;
         if (least >= dev::kInfBits) {
           converged = true;
