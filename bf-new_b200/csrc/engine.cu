@@ -393,13 +393,25 @@ __device__ __forceinline__ void jacobi_item(const LaunchParams& p, const DBatch&
     if ((vt.x >> ql) & 1u) {
       const u32 cb = __ldg(p.g.csc_off + v), ce = __ldg(p.g.csc_off + v + 1);
       if (kCount) wk.c[8] += ce - cb;
-      for (u32 e = cb; e < ce; ++e) {
-        const uint4 rec = __ldg(p.g.csc + e);
-        const uint2 su = B.tiles[rec.w];
-        if ((su.x >> ql) & 1u) {
-          const u32 sb = dev::hi(dev::ld_cg(dr + ((static_cast<u64>(rec.x - su.y) << B.shift) + ql)));
-          if (sb != dev::kInfBits) {
-            const u64 cand = dev::candidate(sb, rec.y, rec.z);
+      // four in-edges at a time: their records, tile entries and labels are
+      // each read together, so an item waits three times per four edges
+      for (u32 e = cb; e < ce; e += 4u) {
+        uint4 rec[4];
+        u32 sb[4];
+#pragma unroll
+        for (u32 k = 0; k < 4u; ++k) rec[k] = __ldg(p.g.csc + min(e + k, ce - 1u));
+#pragma unroll
+        for (u32 k = 0; k < 4u; ++k) {
+          const uint2 su = B.tiles[rec[k].w];
+          sb[k] = dev::kInfBits;
+          if (e + k < ce && ((su.x >> ql) & 1u)) {
+            sb[k] = dev::hi(dev::ld_cg(dr + ((static_cast<u64>(rec[k].x - su.y) << B.shift) + ql)));
+          }
+        }
+#pragma unroll
+        for (u32 k = 0; k < 4u; ++k) {
+          if (sb[k] != dev::kInfBits) {
+            const u64 cand = dev::candidate(sb[k], rec[k].y, rec[k].z);
             best = cand < best ? cand : best;
             if (kCount) wk.c[9] += 1;
           }
@@ -440,17 +452,30 @@ __device__ __forceinline__ void dense_item(const LaunchParams& p, const DBatch& 
           wk.c[1] += re - rb;
           wk.c[2] += 1;
         }
-        for (u32 e = rb; e < re; ++e) {
-          const uint4 rec = __ldg(p.g.csr + e);
-          const uint2 dt = B.tiles[rec.w];
-          if ((dt.x >> ql) & 1u) {
-            const u64 cand = dev::candidate(sb, rec.y, rec.z);
-            u64* const target = B.dist[0] + ((static_cast<u64>(rec.x - dt.y) << B.shift) + ql);
-            const u64 cur = dev::ld_cg(target);
-            if (kCount) wk.c[3] += 1;
-            if (cand < cur) {
-              dev::red_min(target, cand);
-              const bool dec = dev::hi(cand) < dev::hi(cur);
+        // four out-edges at a time, as the pull's in-edges
+        for (u32 e = rb; e < re; e += 4u) {
+          uint4 rec[4];
+          u64* target[4];
+          u64 cur[4];
+#pragma unroll
+          for (u32 k = 0; k < 4u; ++k) rec[k] = __ldg(p.g.csr + min(e + k, re - 1u));
+#pragma unroll
+          for (u32 k = 0; k < 4u; ++k) {
+            const uint2 dt = B.tiles[rec[k].w];
+            target[k] = nullptr;
+            cur[k] = 0u;
+            if (e + k < re && ((dt.x >> ql) & 1u)) {
+              target[k] = B.dist[0] + ((static_cast<u64>(rec[k].x - dt.y) << B.shift) + ql);
+              cur[k] = dev::ld_cg(target[k]);
+              if (kCount) wk.c[3] += 1;
+            }
+          }
+#pragma unroll
+          for (u32 k = 0; k < 4u; ++k) {
+            const u64 cand = dev::candidate(sb, rec[k].y, rec[k].z);
+            if (target[k] != nullptr && cand < cur[k]) {
+              dev::red_min(target[k], cand);
+              const bool dec = dev::hi(cand) < dev::hi(cur[k]);
               if (dec) changed = 1u << ql;
               if (kCount) {
                 wk.c[6] += 1;
