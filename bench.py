@@ -504,7 +504,13 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
     achieved = alg_bytes / (kernel_avg / 1000) / 1e9
     engines_for_step = engines_chosen or [2 if engine_id == bfx.ENGINE_FRONTIER_PUSH else engine_id] * len(descs)
     step = step_label(engines_for_step, deltas, mean_w)
-    if frontier_used == "chunked":
+    # the library's defaults relax lanes in clusters and teams of blocks; the
+    # grid-wide chunked kernel runs where an option of its own is set
+    off_grid = (frontier_used == "chunked" and args.regs == 0 and args.items == 2 and not args.amin
+                and not args.edge_major and not args.pairs)
+    if off_grid:
+        traffic, traffic_source, random_ceiling = None, "no capture of the cluster and team kernels is scaled", None
+    elif frontier_used == "chunked":
         traffic, traffic_source, random_ceiling = traffic_estimate(wl.name, work["relaxations"], kernel_avg, step)
     else:  # the committed traffic captures are of the chunked kernel
         traffic, traffic_source, random_ceiling = None, f"no capture of the {frontier_used} kernel is scaled", None
@@ -523,7 +529,7 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
                    "frontier_layout": frontier_used,
                    "tile_visit_batches": (sum(1 for m in tuned_mappings if m == bfx.MAPPING_TILE_VISITS)
                                           if frontier_used == "tiled" else 0),
-                   "registers": eff_regs, "flat_items": args.items,
+                   "registers": 64 if off_grid else eff_regs, "flat_items": args.items,
                    "returning_min": args.amin, "edge_major": args.edge_major, "chunk_pairs": args.pairs,
                    "chunk_pack": ws.chunk_pack(),
                    "engines_chosen": None if engines_chosen is None else
@@ -542,8 +548,9 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "traffic_source": traffic_source, "peak_source": peak_src,
                      "random_sector_ceiling": random_ceiling, "kernel": "%s (%s frontier, %d registers%s)" % (
+                         "resident_kernel and team_kernel" if off_grid else
                          "persistent_tiled_kernel" if frontier_used == "tiled" else "persistent_kernel",
-                         frontier_used, eff_regs,
+                         frontier_used, 64 if off_grid else eff_regs,
                          ", mixed engines" if engines_chosen and any(e != 2 for e in engines_chosen) else ""),
                      "kernel_ms": kernel_avg, "execute_ms": float(np.mean(execute_ms)),
                      "algorithmic_bytes_per_launch": alg_bytes, "work": work, "engine_work": engine_work},
