@@ -63,7 +63,7 @@ constexpr u32 kShapeCount = sizeof(kShapes) / sizeof(kShapes[0]);
 // Nets that leave SMs idle are spread over larger shapes, up to 8 blocks and
 // at least 64 words (2,048 vertices) a block: below that a round is its fixed
 // latency (one 4,096-vertex net: 0.10 ms on 4 blocks, 0.23 ms on one).
-constexpr size_t kLaunchStreams = 4;
+constexpr size_t kLaunchStreams = 8;
 constexpr u64 kTeamBytes = u64{270} << 20;
 constexpr u32 kSpreadShape = 7u, kSpreadWords = 64u;
 
