@@ -18,7 +18,9 @@
 //     masks are materialised;
 //   * edges are 16-byte records {endpoint, weight bits, eid+1, endpoint tile}
 //     read with 128-bit non-coherent loads;
-//   * the frontier is a queue of 32-vertex chunks by default (frontier.cuh:
+//   * by default a frontier lane is searched on its own, by a cluster or a team
+//     of blocks (resident.cu); what remains takes the grid-wide rounds below;
+//   * the grid-wide frontier is a queue of 32-vertex chunks (frontier.cuh:
 //     chunk bitmaps per round slot, pending lanes set with non-returning ORs,
 //     near and far claims staged per warp and (round, batch)); a warp item
 //     is a pack of up to 8 chunks whose pending vertices are compacted into
@@ -1298,6 +1300,7 @@ int bfx_resident_graph_upload(const bfx_device_graph_layout32* layout, int devic
     BFX_CUDA(cudaMemcpy(base + o_row, csr_row.data(), size_t{V} * 8, cudaMemcpyHostToDevice));
     double wsum = 0.0;
     for (std::uint32_t e = 0; e < E; ++e) wsum += L.csr_weights[e];
+    G->image_host.reserve(bfx::kPieceBytes * bfx::kPieceThreads);
     G->mean_weight = E ? wsum / E : 0.0;
     G->current_mean = G->mean_weight;
     G->g.V = V;
@@ -1994,37 +1997,37 @@ const void* persistent_entry(bool count, std::uint32_t registers, std::uint32_t 
 }  // namespace
 
 // Copies images from the device to pageable host memory (null: not wanted)
-// through a pinned buffer of the workspace, in pieces: the
-// copy out of the pinned piece -- with a page fault per 4 KB of a fresh host
-// array -- takes far longer than the transfer, so from 2 MB on several threads
-// take pieces.  Ends with the stream's work done.  B200 box, one net's image of
-// 65,536 vertices: 0.55 -> 0.1 ms against an asynchronous allocation and two
-// pageable copies.
+// through the graph's pinned pieces (pinning takes milliseconds, so it is done
+// once per graph and not per workspace).  The copy out of a piece -- with a
+// page fault per 4 KB of a fresh host array -- takes far longer than the
+// transfer, so from four pieces on several threads take them.  Ends with the
+// stream's work done; workspaces of one graph take turns, after their streams
+// are idle.  B200, one net's image of 65,536 vertices: 0.56 -> 0.08 ms
+// against an allocation per call and two pageable copies.
 void fetch_images(bfx_workspace* ws, std::initializer_list<HostImage> images) {
-  constexpr size_t kPiece = 512 * 1024;
   struct Piece {
     const char* device;
     char* host;
     size_t bytes;
   };
   std::vector<Piece> pieces;
-  size_t largest = 0;
   for (const HostImage& im : images) {
     if (im.host == nullptr) continue;
-    for (size_t at = 0; at < im.bytes; at += kPiece) {
+    for (size_t at = 0; at < im.bytes; at += kPieceBytes) {
       pieces.push_back({static_cast<const char*>(im.device) + at, static_cast<char*>(im.host) + at,
-                        std::min(kPiece, im.bytes - at)});
-      largest = std::max(largest, pieces.back().bytes);
+                        std::min(kPieceBytes, im.bytes - at)});
     }
   }
   const unsigned threads =
-      pieces.size() < 4 ? 1U : std::min<unsigned>({4U, std::max(1U, std::thread::hardware_concurrency()),
+      pieces.size() < 4 ? 1U : std::min<unsigned>({kPieceThreads, std::max(1U, std::thread::hardware_concurrency()),
                                                    static_cast<unsigned>(pieces.size())});
-  ws->image_host.reserve(threads * largest + 1);
+  BFX_CUDA(cudaStreamSynchronize(ws->stream));
+  std::lock_guard<std::mutex> lock(ws->graph->image_mutex);
+  char* const buffer = static_cast<char*>(ws->graph->image_host.ptr);
   std::atomic<size_t> next{0};
   std::atomic<int> error{cudaSuccess};
   const auto work = [&](unsigned t) {
-    char* const pinned = static_cast<char*>(ws->image_host.ptr) + t * largest;
+    char* const pinned = buffer + t * kPieceBytes;
     if (t != 0U) {
       const cudaError_t e = cudaSetDevice(ws->graph->device);
       if (e != cudaSuccess) error = e;

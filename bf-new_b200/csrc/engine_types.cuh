@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cstring>
 #include <initializer_list>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -273,6 +274,9 @@ struct bfx_resident_graph {
   // dealt to blocks in runs of 2^word_run; word_whole: every tile is one run.
   std::uint32_t word_run{3};
   bool word_whole{false};
+  // Pinned pieces of downloads (fetch_images), one download at a time.
+  std::mutex image_mutex;
+  bfx::PinnedBuffer image_host;
   std::uint32_t resident_shapes{0};  // block configurations that the device holds
 };
 
@@ -289,7 +293,6 @@ struct bfx_workspace {
   bfx::DeviceBuffer tile_tables;  // per batch dense {lane mask, compact bias} over all tiles
   bfx::DeviceBuffer qimage;       // device-side preparation: the uploaded query and lane image
   bfx::DeviceBuffer image;        // label images and path payloads on their way to the host
-  bfx::PinnedBuffer image_host;
   bfx::PinnedBuffer staging;
   bfx::PinnedBuffer status_host;
   size_t meta_bytes{0};
@@ -357,6 +360,9 @@ namespace bfx {
 
 // Device bytes of a download at a time, at most.
 constexpr size_t kImageBytes = size_t{64} << 20;
+// Its pinned pieces, one per thread.
+constexpr size_t kPieceBytes = size_t{512} << 10;
+constexpr unsigned kPieceThreads = 4;
 
 struct HostImage {
   const void* device;
