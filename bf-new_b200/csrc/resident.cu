@@ -82,20 +82,23 @@ __device__ __forceinline__ u32 map_rank(u32 address, u32 rank) {
   return r;
 }
 // Loads and reductions by shared-memory address: here: in the own block, else
-// in any block of the cluster (kCluster).  Both forms are predicated, not
-// branched to, so the loads of several edges are in flight together.
+// in any block of the cluster (kCluster).  Neighbours lower the same words at
+// the same time, so in a cluster both forms have cluster scope: two accesses
+// whose scopes do not include each other's thread would not be atomic to one
+// another.  Both are predicated, not branched to, so the loads of several
+// edges are in flight together.
 template <bool kCluster>
 __device__ __forceinline__ u32 shared_load(u32 a, bool here) {
   u32 v;
   if (kCluster) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
-        "@p ld.volatile.shared.u32 %0, [%1];\n\t@!p ld.relaxed.cluster.shared::cluster.u32 %0, [%1];\n\t}"
+        "@p ld.relaxed.cluster.shared::cta.u32 %0, [%1];\n\t@!p ld.relaxed.cluster.shared::cluster.u32 %0, [%1];\n\t}"
         : "=r"(v)
         : "r"(a), "r"(static_cast<u32>(here))
         : "memory");
   } else {
-    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    asm volatile("ld.relaxed.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
   }
   return v;
 }
@@ -104,11 +107,12 @@ __device__ __forceinline__ void shared_min(u32 a, u32 v, bool here) {
   if (kCluster) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
-        "@p red.relaxed.cta.shared.min.u32 [%0], %1;\n\t@!p red.relaxed.cluster.shared::cluster.min.u32 [%0], %1;\n\t}"
-        ::"r"(a), "r"(v), "r"(static_cast<u32>(here))
+        "@p red.relaxed.cluster.shared::cta.min.u32 [%0], %1;\n\t"
+        "@!p red.relaxed.cluster.shared::cluster.min.u32 [%0], %1;\n\t}" ::"r"(a),
+        "r"(v), "r"(static_cast<u32>(here))
         : "memory");
   } else {
-    asm volatile("red.relaxed.cta.shared.min.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    asm volatile("red.relaxed.cta.shared::cta.min.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
   }
 }
 template <bool kCluster>
@@ -116,11 +120,12 @@ __device__ __forceinline__ void shared_or(u32 a, u32 v, bool here) {
   if (kCluster) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
-        "@p red.relaxed.cta.shared.or.b32 [%0], %1;\n\t@!p red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;\n\t}"
-        ::"r"(a), "r"(v), "r"(static_cast<u32>(here))
+        "@p red.relaxed.cluster.shared::cta.or.b32 [%0], %1;\n\t"
+        "@!p red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;\n\t}" ::"r"(a),
+        "r"(v), "r"(static_cast<u32>(here))
         : "memory");
   } else {
-    asm volatile("red.relaxed.cta.shared.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    asm volatile("red.relaxed.cta.shared::cta.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
   }
 }
 __device__ __forceinline__ void remote_store(u32 a, u32 v) {
@@ -394,7 +399,7 @@ __global__ void __launch_bounds__(1024, 1)
     const auto relax = [&](u32 slot, u32 v, uint2 row, u32 take) {
       u32 d = dev::kInfBits, so = 0u, tile = kFull;
       if (lane < take) {
-        d = L[slot];
+        d = shared_load<kCluster>(L_at + slot * 4u, true);  // neighbours may be lowering it
         so = slot - v;
         tile = gtile[slot >> 5];
         if (kCount) {
