@@ -642,6 +642,11 @@ class Workspace:
         whole-graph lanes by a team of blocks each; 0: every lane takes the grid-wide kernels."""
         _check(load().bfx_set_resident_nets(self._h, u32(mode)))
 
+    def set_launch_budget(self, nanoseconds: int):
+        """Wall-clock budget of a relaxation (1 ns .. 30 s, the default); past it the batches report a device
+        failure and the workspace stays usable."""
+        _check(load().bfx_set_launch_budget(self._h, u64(nanoseconds)))
+
     def set_chunk_pairs(self, mode: int):
         """Chunked layout: 0 work list, 1 (vertex, lane) pair per thread (persistent control)."""
         _check(load().bfx_set_chunk_pairs(self._h, u32(mode)))

@@ -2083,7 +2083,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
   p.engine = o.engine;
   p.per_lane = o.enable_per_lane_convergence;
   p.max_rounds = o.maximum_rounds;
-  p.budget_ns = kLaunchBudgetNs;
+  p.budget_ns = ws->budget_ns;
   p.engines = nullptr;
   p.deltas = nullptr;
   const float auto_step = kAutoSteps * static_cast<float>(ws->graph->current_mean);
@@ -2253,7 +2253,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
       BFX_CUDA(cudaStreamSynchronize(ws->stream));
       ++ws->last_host_checks;
       if (*done_host) break;
-      if (std::chrono::steady_clock::now() - t0 > std::chrono::nanoseconds(kLaunchBudgetNs)) {
+      if (std::chrono::steady_clock::now() - t0 > std::chrono::nanoseconds(ws->budget_ns)) {
         // same outcome as a persistent launch past its budget: device_failure
         BFX_CUDA(cudaMemsetAsync(&p.run->abort, 1, 1, ws->stream));
         break;
@@ -2289,6 +2289,14 @@ int bfx_set_resident_nets(bfx_workspace* ws, uint32_t mode) {
     bfx::require(ws != nullptr, "null argument");
     bfx::require(mode <= 1u, "resident nets must be 0 or 1");
     ws->resident_mode = mode;
+  });
+}
+
+int bfx_set_launch_budget(bfx_workspace* ws, uint64_t nanoseconds) {
+  return bfx::guarded([&] {
+    bfx::require(ws != nullptr, "null argument");
+    bfx::require(nanoseconds >= 1u && nanoseconds <= bfx::kLaunchBudgetNs, "launch budget must be 1 ns .. 30 s");
+    ws->budget_ns = nanoseconds;
   });
 }
 

@@ -334,6 +334,7 @@ struct bfx_workspace {
   bfx::TeamState* d_teams{nullptr};
   const bfx::u32* d_fit{nullptr};
   std::uint32_t resident_mode = 1;   // see bfx_set_resident_nets
+  std::uint64_t budget_ns = bfx::kLaunchBudgetNs;  // see bfx_set_launch_budget
   cudaEvent_t resident_fork{nullptr};
   std::vector<cudaStream_t> resident_streams;
   std::vector<cudaEvent_t> resident_joins;

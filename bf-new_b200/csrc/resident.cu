@@ -262,8 +262,7 @@ __global__ void __launch_bounds__(1024, 1)
   const ResidentNet net = nets[blockIdx.x / ctas];
   const u32 b = net.batch, ql = net.lane;
   const u32 rank = kCluster ? cluster_rank() : 0u;
-  // uniform over the cluster: the batch's engine, and a launch already past
-  // its budget (read once, before any barrier, by every block)
+  // uniform over the cluster
   if (engine_of(p, b) != BFX_ENGINE_FRONTIER_PUSH) return;
   const DBatch& B = p.batches[b];
   DCtl& C = p.ctl[b];
@@ -529,8 +528,11 @@ __global__ void __launch_bounds__(1024, 1)
       }
     }
     if (__any_sync(kFull, any) && lane < ctas) remote_store(map_rank(shared_address(&s.any[rounds % 3u]), lane), 1u);
-    if ((rounds & 255u) == 255u && tid < ctas && rank == 0u && dev::global_ns() - t0 > p.budget_ns) {
-      remote_store(map_rank(shared_address(&s.stop), tid), 1u);
+    if ((rounds & 255u) == 255u && rank == 0u && warp == 0u) {
+      // one thread's clock decides for the whole cluster: blocks that left at
+      // different rounds would wait for, or read, blocks that are gone
+      const bool over = lane == 0u && dev::global_ns() - t0 > p.budget_ns;
+      if (__shfl_sync(kFull, over, 0) && lane < ctas) remote_store(map_rank(shared_address(&s.stop), lane), 1u);
     }
     cluster_sync(ctas);
     const bool more = s.any[rounds % 3u] != 0u;

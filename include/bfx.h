@@ -362,6 +362,10 @@ int bfx_get_frontier_mapping(bfx_workspace *ws, uint32_t *layout, uint32_t count
  * _flat_items, _flat_order, _relax_atomic, _chunk_pairs) stay grid-wide.  The
  * round count of a batch is then the largest of its lanes'. */
 int bfx_set_resident_nets(bfx_workspace *ws, uint32_t mode);
+/* Wall-clock budget of a relaxation, 1 ns .. 30 s (the default).  The kernels
+ * look at it every few rounds; a launch past it stops and its batches report
+ * BFX_STOP_DEVICE_FAILURE, the workspace stays usable (bfx extension). */
+int bfx_set_launch_budget(bfx_workspace *ws, uint64_t nanoseconds);
 /* Register budget of the persistent relaxation kernel (a bfx tuning option,
  * results unchanged): 40 registers per thread (three 512-thread blocks per
  * SM), 64 (two 512-thread blocks per SM: no spills in the group layout, few

@@ -1,0 +1,59 @@
+"""Limits of a relaxation: a spent wall-clock budget ends every search the
+normal way, with a status that says so and a workspace that stays usable."""
+import numpy as np
+import pytest
+
+import bfx
+
+pytestmark = pytest.mark.gpu
+
+
+def chain(n, tile=128):
+    """Vertices 0 .. n-1 in tiles of `tile`, edges i -> i+1 of weight 1: the
+    search from vertex 0 takes n rounds and reaches n-1 at distance n-1."""
+    i = np.arange(n)
+    e = n - 1
+    g = bfx.InputGraph(i // tile, np.zeros(n), np.ones(n), np.zeros(n), i[:-1], i[1:], np.ones(e), np.zeros(e),
+                       np.zeros(e), np.arange(e))
+    layout = bfx.build_device_graph_layout(g, bfx.SpatialOrderConfig(0, 0, 1, 1))
+    order = np.argsort(layout.tiles["new_to_old"])  # old vertex -> new
+    q = bfx.RouteQuery(1, [int(order[0])], [int(order[n - 1])], np.arange(layout.tile_count))
+    return layout, bfx.make_description(layout, [q], 1), order
+
+
+def prepared(layout, desc):
+    resident = bfx.ResidentDeviceGraph.upload_once(layout)
+    ws = bfx.Workspace(resident)
+    ws.prepare([desc])
+    ws.set_batch_deltas([np.inf])
+    return resident, ws
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [2_000, 3_000, 20_000, 450_000, 600_000, 900_000])
+def test_spent_budget_stops_every_search(gpu, n, mode):
+    """One block, clusters of 2 to 16 blocks, a team and the grid-wide kernel:
+    a cluster's blocks stop in the same round, or they would wait for one
+    another."""
+    layout, desc, order = chain(n)
+    resident, ws = prepared(layout, desc)
+    ws.set_resident_nets(mode)
+    ws.set_launch_budget(1)
+    ws.execute(bfx.GpuRunOptions())
+    (st,) = ws.fetch_statuses()
+    assert st.stop_reason == bfx.STOP_FAILURE and st.converged == 0
+    assert st.rounds_completed <= 256
+    ws.set_launch_budget(30_000_000_000)
+    if n <= 20_000:
+        ws.execute(bfx.GpuRunOptions())
+        (st,) = ws.fetch_statuses()
+        assert st.stop_reason == bfx.STOP_CONVERGED
+        assert ws.download_lane(0, 0)[0].view(np.float32)[order[n - 1]] == n - 1
+    else:
+        ws.execute(bfx.GpuRunOptions(maximum_rounds=2))
+        assert ws.fetch_statuses()[0].stop_reason == bfx.STOP_MAXIMUM_ROUNDS
+    for bad in (0, 30_000_000_001):
+        with pytest.raises(ValueError):
+            ws.set_launch_budget(bad)
+    ws.close()
+    resident.close()
