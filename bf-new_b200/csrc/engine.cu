@@ -310,6 +310,7 @@ __global__ void init_kernel(LaunchParams p) {
     p.run->done = 0u;
     p.run->stop = 0u;
     p.run->abort = 0u;
+    p.run->started = dev::global_ns();
     for (int i = 0; i < 16; ++i) p.run->work[i] = 0u;
     for (int i = 0; i < 3; ++i) p.run->items[i] = 0u;
   }

@@ -106,8 +106,7 @@ struct DRun {
   u32 done;        // all batches stopped
   u32 stop;        // launch-wide stop reason
   u32 abort;       // device failure seen
-  u64 max_rounds;
-  u64 launches;
+  u64 started;     // %globaltimer when the relaxation began: what its searches' budget counts from
   u64 work[16];    // launch-wide work counters: [0..6] push engines, [7] rounds, [8..11] Jacobi, [12..13] splits,
                    // [14..15] tiled visits (lane-edge relaxations inside shared memory, staged visits)
   u32 items[3];    // tiled layout: block items drawn in round r from items[r % 3] (cleared two rounds ahead)
@@ -135,7 +134,7 @@ struct Work {
 
 constexpr u32 kMaxBatchesPerLaunch = 4096;
 constexpr u64 kBarrierTimeoutNs = 2000000000ull;  // 2 s per barrier wait
-constexpr u64 kLaunchBudgetNs = 30000000000ull;   // 30 s per relaxation launch
+constexpr u64 kLaunchBudgetNs = 30000000000ull;   // 30 s per relaxation: all launches of one execute
 
 // Searches that find predecessors after convergence (resident.cu) need at
 // least this round limit: a launch that stops on its
@@ -160,7 +159,7 @@ struct LaunchParams {
   u32 flat;              // frontier layout: 0 sub-warp groups, 1 flat work list, 2 chunked flat work list,
                          // 3 tiled (a block visits 2^cshift compact vertices with their labels in shared memory)
   u64 max_rounds;
-  u64 budget_ns;         // wall-clock budget of one relaxation launch; past it the launch stops (device_failure)
+  u64 budget_ns;         // wall-clock budget of the relaxation; past it its launches stop (device_failure)
   const u32* engines;    // [nb] per-batch engine (autotuned launches) or null
   const u32* deltas;     // [nb] near/far threshold steps (float bits) or null (plain frontier)
   u32 auto_step;         // step of the searches of resident.cu where `deltas` is null (float bits): kAutoSteps

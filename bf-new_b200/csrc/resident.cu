@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(1024, 1)
     return Place{q - deal * ctas, (((deal << run) | (w & run_mask)) << 5) | (idx & 31u)};
   };
   const u32 L_at = shared_address(L);
-  const u64 t0 = dev::global_ns();
+  const u64 t0 = p.run->started;  // the budget is the relaxation's, however long the search was queued
 
   // --- the net's tiles and words -------------------------------------------
   for (u32 i = tid; i < dw; i += blockDim.x) dir[i] = make_uint2(0u, 0u);
@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(1024, 1)
       }
     }
     if (__any_sync(kFull, any) && lane < ctas) remote_store(map_rank(shared_address(&s.any[rounds % 3u]), lane), 1u);
-    if ((rounds & 255u) == 255u && rank == 0u && warp == 0u) {
+    if ((rounds & 255u) == 0u && rank == 0u && warp == 0u) {
       // one thread's clock decides for the whole cluster: blocks that left at
       // different rounds would wait for, or read, blocks that are gone
       const bool over = lane == 0u && dev::global_ns() - t0 > p.budget_ns;
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(1024, 1)
   TeamState& S = states[team];
   const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, warps = blockDim.x >> 5;
   const u32 V = p.g.V, words = (V + 31u) >> 5;
-  const u64 t0 = dev::global_ns();
+  const u64 t0 = p.run->started;  // the budget is the relaxation's, however long the search was queued
   if (tid < 2u) {
     s_listed[tid] = 0u;
     s_cut[tid] = kFull;
@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(1024, 1)
       }
       ++pass;
       if (__syncthreads_or(any) && tid == 0u) atomicExch(&S.any[r % 3u], 1u);
-      if ((r & 63u) == 63u && rank == 0u && tid == 0u && dev::global_ns() - t0 > p.budget_ns) {
+      if ((r & 63u) == 0u && rank == 0u && tid == 0u && dev::global_ns() - t0 > p.budget_ns) {
         atomicExch(&S.sync.abort, 1u);
       }
       if (!barrier()) return;

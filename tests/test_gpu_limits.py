@@ -57,3 +57,27 @@ def test_spent_budget_stops_every_search(gpu, n, mode):
             ws.set_launch_budget(bad)
     ws.close()
     resident.close()
+
+
+def test_budget_covers_queued_searches(gpu):
+    """More searches than run at once: each alone is well within the budget,
+    all of them one after another are not."""
+    layout, _, order = chain(20_000)
+    first, last = int(order[0]), int(order[-1])
+    queries = [bfx.RouteQuery(k, [first], [last], np.arange(layout.tile_count)) for k in range(32)]
+    desc = bfx.make_description(layout, queries, 32)
+    resident = bfx.ResidentDeviceGraph.upload_once(layout)
+    ws = bfx.Workspace(resident)
+    ws.prepare([desc] * 40)
+    ws.execute(bfx.GpuRunOptions())
+    assert all(st.stop_reason == bfx.STOP_CONVERGED for st in ws.fetch_statuses())
+    together = ws.last_execute_timing()[0] * 1e6
+    ws.set_launch_budget(int(0.6 * together))
+    ws.execute(bfx.GpuRunOptions())
+    assert all(st.stop_reason == bfx.STOP_FAILURE for st in ws.fetch_statuses())
+    ws.prepare([desc])
+    ws.execute(bfx.GpuRunOptions())
+    assert ws.last_execute_timing()[0] * 1e6 < 0.6 * together
+    assert ws.fetch_statuses()[0].stop_reason == bfx.STOP_CONVERGED
+    ws.close()
+    resident.close()
