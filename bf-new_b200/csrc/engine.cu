@@ -1560,6 +1560,8 @@ Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector
   }
   ubase[count] = static_cast<std::uint32_t>(usum);
   sbase[count] = static_cast<std::uint32_t>(ssum);
+  ws->search_rounds = whole.empty() ? 0u : g.V;
+  if (!nets.empty()) ws->search_rounds = std::max(ws->search_rounds, u64{nets[0].words} * 32u);  // largest first
   for (const ResidentNet& n : whole) ws->batches[n.batch].team = 1u;
   std::memcpy(hb + o_batch, ws->batches.data(), count * sizeof(DBatch));
   if (!whole.empty()) std::memcpy(hb + o_whole, whole.data(), whole.size() * sizeof(ResidentNet));
@@ -2135,14 +2137,13 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
   }
   // Frontier lanes that fit a cluster's shared memory are relaxed there
   // (resident.cu); what remains takes the grid-wide kernels.  Not for launches
-  // that may stop on their round limit (its labels carry no predecessors
-  // until they converge), that trace rounds, or that set a grid, a layout or
-  // an option of the grid-wide kernels.
+  // that may stop on their round limit (kLateRounds), that trace rounds, or
+  // that set a grid, a layout or an option of the grid-wide kernels.
   const bool resident = ws->resident_mode != 0u && !(ws->nets.empty() && ws->whole.empty()) && p.flat == 2u &&
                         ws->frontier_layout == BFX_FRONTIER_CHUNKED && p.engine == BFX_ENGINE_FRONTIER_PUSH &&
-                        o.maximum_rounds >= kLateRounds && o.instrumentation < 2u && o.grid_policy == 0u &&
-                        ws->relax_atomic == 0u && ws->edge_major == 0u && ws->chunk_pairs == 0u &&
-                        ws->flat_items == 2u && ws->register_budget == 0u;
+                        o.maximum_rounds >= std::max(kLateRounds, ws->search_rounds) && o.instrumentation < 2u &&
+                        o.grid_policy == 0u && ws->relax_atomic == 0u && ws->edge_major == 0u &&
+                        ws->chunk_pairs == 0u && ws->flat_items == 2u && ws->register_budget == 0u;
   bool remaining = !resident;
   if (resident) {
     p.fit = ws->d_fit;

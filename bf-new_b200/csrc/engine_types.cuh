@@ -136,9 +136,13 @@ constexpr u32 kMaxBatchesPerLaunch = 4096;
 constexpr u64 kBarrierTimeoutNs = 2000000000ull;  // 2 s per barrier wait
 constexpr u64 kLaunchBudgetNs = 30000000000ull;   // 30 s per relaxation: all launches of one execute
 
-// Searches that find predecessors after convergence (resident.cu) need at
-// least this round limit: a launch that stops on its
-// limit reports labels mid-way.
+// Searches that find predecessors after convergence (resident.cu) must not
+// stop on a round limit: a launch that does reports labels mid-way.  A search
+// never takes more rounds than its lane has vertices: the k-th round after a
+// split settles, along every shortest path, the k-th vertex below the
+// threshold, a split moves at least one such vertex, and each is settled once.
+// So they run under limits above the vertices of the set's largest lane, and
+// from this limit on.
 constexpr u64 kLateRounds = 65536u;
 
 // Near/far step of a set that was given none, in mean edge weights.  Plain
@@ -332,6 +336,7 @@ struct bfx_workspace {
   const bfx::ResidentNet* d_whole{nullptr};
   bfx::TeamState* d_teams{nullptr};
   const bfx::u32* d_fit{nullptr};
+  std::uint64_t search_rounds{0};    // no search of the prepared set takes more rounds (at least its largest lane's vertices)
   std::uint32_t resident_mode = 1;   // see bfx_set_resident_nets
   std::uint64_t budget_ns = bfx::kLaunchBudgetNs;  // see bfx_set_launch_budget
   cudaEvent_t resident_fork{nullptr};

@@ -357,8 +357,9 @@ int bfx_get_frontier_mapping(bfx_workspace *ws, uint32_t *layout, uint32_t count
  * thread-block cluster is relaxed by a cluster of its own, and each larger
  * whole-graph lane by a team of thread blocks, outside the grid-wide kernels;
  * 0 relaxes every lane grid-wide.  Launches that set
- * maximum_rounds below 65,536, an explicit grid, round tracing, another
- * frontier layout or an option of the grid-wide kernels (bfx_set_register_budget,
+ * maximum_rounds below 65,536 or below the vertices of the set's largest lane
+ * (each tile rounded up to 32; no search takes more rounds, so none stops on
+ * its limit), an explicit grid, round tracing, another frontier layout or an option of the grid-wide kernels (bfx_set_register_budget,
  * _flat_items, _flat_order, _relax_atomic, _chunk_pairs) stay grid-wide.  The
  * round count of a batch is then the largest of its lanes'. */
 int bfx_set_resident_nets(bfx_workspace *ws, uint32_t mode);

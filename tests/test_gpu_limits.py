@@ -1,5 +1,6 @@
 """Limits of a relaxation: a spent wall-clock budget ends every search the
-normal way, with a status that says so and a workspace that stays usable."""
+normal way, with a status that says so and a workspace that stays usable, and a
+round limit that a search could reach is kept exactly."""
 import numpy as np
 import pytest
 
@@ -79,5 +80,31 @@ def test_budget_covers_queued_searches(gpu):
     ws.execute(bfx.GpuRunOptions())
     assert ws.last_execute_timing()[0] * 1e6 < 0.6 * together
     assert ws.fetch_statuses()[0].stop_reason == bfx.STOP_CONVERGED
+    ws.close()
+    resident.close()
+
+
+@pytest.mark.parametrize("limit,stop", [(65_536, "limit"), (69_999, "limit"), (70_000, "converged"),
+                                        (70_100, "converged"), (1 << 40, "converged")])
+def test_round_limit_that_a_search_can_reach(gpu, limit, stop):
+    """A chain of 70,000 vertices takes 70,000 rounds (the last finds nothing
+    to improve): limits below it stop the run there, whatever kernel would
+    take the lane."""
+    n = 70_000
+    layout, desc, order = chain(n)
+    resident, ws = prepared(layout, desc)
+    ws.execute(bfx.GpuRunOptions(maximum_rounds=limit))
+    (st,) = ws.fetch_statuses()
+    bits, pred = ws.download_lane(0, 0)
+    distance = bits.view(np.float32)[order]
+    if stop == "converged":
+        assert st.stop_reason == bfx.STOP_CONVERGED and st.rounds_completed <= limit
+        np.testing.assert_array_equal(distance, np.arange(n))
+    else:
+        assert st.stop_reason == bfx.STOP_MAXIMUM_ROUNDS and st.rounds_completed == limit
+        assert st.converged == 0 and st.active_lane_mask == 1
+        np.testing.assert_array_equal(distance[:limit + 1], np.arange(limit + 1))
+        assert np.all(np.isinf(distance[limit + 1:]))
+        assert np.all(pred[order[1:limit + 1]] != 0xFFFFFFFF)
     ws.close()
     resident.close()
