@@ -6,6 +6,7 @@
 #include "bfx.h"
 #include "bfx_internal.hpp"
 #include "device_common.cuh"
+#include "side_streams.hpp"
 
 #include <cuda_runtime.h>
 
@@ -211,6 +212,14 @@ __device__ __forceinline__ u32 engine_of(const LaunchParams& p, u32 b) {
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t{255}; }
 
+struct CudaStreams {
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
+  static void record(Event event, Stream stream) { BFX_CUDA(cudaEventRecord(event, stream)); }
+  static void wait(Stream stream, Event event) { BFX_CUDA(cudaStreamWaitEvent(stream, event, 0)); }
+  static void synchronize(Stream stream) noexcept { cudaStreamSynchronize(stream); }
+};
+
 struct DeviceBuffer {
   void* ptr{nullptr};
   size_t bytes{0};
@@ -340,8 +349,7 @@ struct bfx_workspace {
   std::uint32_t resident_mode = 1;   // see bfx_set_resident_nets
   std::uint64_t budget_ns = bfx::kLaunchBudgetNs;  // see bfx_set_launch_budget
   cudaEvent_t resident_fork{nullptr};
-  std::vector<cudaStream_t> resident_streams;
-  std::vector<cudaEvent_t> resident_joins;
+  std::vector<bfx::SideStreams<bfx::CudaStreams>::Side> resident_sides;
   std::vector<std::uint32_t> batch_engines;  // per-batch engine for BFX_ENGINE_AUTO launches
   std::vector<float> batch_deltas;           // per-batch near/far steps (empty: plain frontier)
   std::vector<std::uint32_t> batch_mappings; // tiled layout: per-batch dense-round mapping (empty: tile visits)

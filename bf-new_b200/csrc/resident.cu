@@ -1243,24 +1243,23 @@ u32 launch_resident(bfx_workspace* ws, const LaunchParams& p, bool count) {
   // The shapes run side by side on up to kLaunchStreams streams in turn,
   // largest first; ws->stream is the first of them.
   const size_t used = std::min<size_t>(groups.size(), kLaunchStreams);
-  while (ws->resident_streams.size() + 1 < used) {
-    cudaStream_t st = nullptr;
-    BFX_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    ws->resident_streams.push_back(st);
-    cudaEvent_t ev = nullptr;
-    BFX_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    ws->resident_joins.push_back(ev);
+  ws->resident_sides.reserve(kLaunchStreams);
+  while (ws->resident_sides.size() + 1 < used) {
+    SideStreams<CudaStreams>::Side side{};
+    BFX_CUDA(cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking));
+    const cudaError_t err = cudaEventCreateWithFlags(&side.done, cudaEventDisableTiming);
+    if (err != cudaSuccess) cudaStreamDestroy(side.stream);
+    BFX_CUDA(err);
+    ws->resident_sides.push_back(side);
   }
-  if (used > 1) {
-    if (!ws->resident_fork) BFX_CUDA(cudaEventCreateWithFlags(&ws->resident_fork, cudaEventDisableTiming));
-    BFX_CUDA(cudaEventRecord(ws->resident_fork, ws->stream));
-    for (size_t i = 1; i < used; ++i) BFX_CUDA(cudaStreamWaitEvent(ws->resident_streams[i - 1], ws->resident_fork, 0));
-  }
+  if (used > 1 && !ws->resident_fork) BFX_CUDA(cudaEventCreateWithFlags(&ws->resident_fork, cudaEventDisableTiming));
+  SideStreams<CudaStreams> sides(ws->stream, ws->resident_fork, ws->resident_sides.data(), used - 1);
   u32 launches = 0;
   for (size_t i = 0; i < groups.size(); ++i) {
     const Shape& sh = kShapes[groups[i].first];
     const u32 first = groups[i].second.first, last = groups[i].second.second;
-    const cudaStream_t stream = i % kLaunchStreams == 0 ? ws->stream : ws->resident_streams[i % kLaunchStreams - 1];
+    const size_t on = i % kLaunchStreams;
+    const cudaStream_t stream = on == 0 ? ws->stream : ws->resident_sides[on - 1].stream;
     size_t bytes = 0;
     for (u32 n = first; n < last; ++n) {
       bytes = std::max(bytes, block_bytes(nets[n].words, nets[n].tiles, sh.ctas, sh.threads, p.g.T, run));
@@ -1284,16 +1283,15 @@ u32 launch_resident(bfx_workspace* ws, const LaunchParams& p, bool count) {
     BFX_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
     ++launches;
   }
-  for (size_t i = 1; i < used; ++i) {
-    BFX_CUDA(cudaEventRecord(ws->resident_joins[i - 1], ws->resident_streams[i - 1]));
-    BFX_CUDA(cudaStreamWaitEvent(ws->stream, ws->resident_joins[i - 1], 0));
-  }
+  sides.join();
   return launches;
 }
 
 void resident_release(bfx_workspace* ws) {
-  for (cudaStream_t st : ws->resident_streams) cudaStreamDestroy(st);
-  for (cudaEvent_t ev : ws->resident_joins) cudaEventDestroy(ev);
+  for (const auto& side : ws->resident_sides) {
+    cudaStreamDestroy(side.stream);
+    cudaEventDestroy(side.done);
+  }
   if (ws->resident_fork) cudaEventDestroy(ws->resident_fork);
 }
 
