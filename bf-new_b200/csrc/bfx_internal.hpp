@@ -97,4 +97,24 @@ void parallel_for(std::uint64_t n, unsigned threads, F&& body) {
   }
 }
 
+// Runs work(0) on this thread and work(1) .. work(n - 1) on threads of their
+// own, and waits for all of them.  Where a thread cannot be had, that one and
+// those after it are left out: the parts of `work` take what there is to do in
+// turn.  On the other threads it must not throw.
+template <typename Thread = std::thread, typename Work>
+void run_together(unsigned n, Work&& work) {
+  struct Pool {
+    std::vector<Thread> threads;
+    ~Pool() {
+      for (auto& t : threads) t.join();
+    }
+  } pool;
+  try {
+    pool.threads.reserve(n);
+    for (unsigned t = 1; t < n; ++t) pool.threads.emplace_back([&work, t] { work(t); });
+  } catch (const std::exception&) {  // std::system_error, std::bad_alloc
+  }
+  work(0U);
+}
+
 }  // namespace bfx

@@ -49,7 +49,6 @@
 #include <memory>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -2046,16 +2045,7 @@ void fetch_images(bfx_workspace* ws, std::initializer_list<HostImage> images) {
       std::memcpy(p.host, pinned, p.bytes);
     }
   };
-  std::vector<std::thread> pool;
-  for (unsigned t = 1; t < threads; ++t) {
-    try {
-      pool.emplace_back(work, t);
-    } catch (const std::system_error&) {
-      break;  // the calling thread takes the rest
-    }
-  }
-  work(0U);
-  for (auto& t : pool) t.join();
+  run_together(threads, work);
   BFX_CUDA(static_cast<cudaError_t>(error.load()));
   BFX_CUDA(cudaStreamSynchronize(ws->stream));
 }
