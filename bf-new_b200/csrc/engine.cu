@@ -1996,35 +1996,53 @@ const void* persistent_entry(bool count, std::uint32_t registers, std::uint32_t 
                : reinterpret_cast<const void*>(persistent_kernel<false, 2, 2>);
 }
 
+// Whether [p, p + bytes) is memory that CUDA knows: page-locked, or managed.
+bool known_memory(const char* p, size_t bytes) {
+  for (const char* at : {p, p + bytes - 1}) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, at) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type == cudaMemoryTypeUnregistered) return false;
+  }
+  return true;
+}
+
 }  // namespace
 
-// Copies images from the device to pageable host memory (null: not wanted)
-// through the graph's pinned pieces (pinning takes milliseconds, so it is done
-// once per graph and not per workspace).  The copy out of a piece -- with a
-// page fault per 4 KB of a fresh host array -- takes far longer than the
-// transfer, so from four pieces on several threads take them.  Ends with the
-// stream's work done; workspaces of one graph take turns, after their streams
-// are idle.  B200, one net's image of 65,536 vertices: 0.56 -> 0.08 ms
-// against an allocation per call and two pageable copies.
+// Copies images from the device to host memory (null: not wanted), and ends
+// with the stream's work done.  Page-locked memory is written by the copy
+// itself.  Pageable memory goes through the graph's pinned pieces (pinning
+// takes milliseconds, so it is done once per graph and not per workspace): the
+// copy out of a piece -- with a page fault per 4 KB of a fresh host array --
+// takes far longer than the transfer, so from four pieces on several threads
+// take them; workspaces of one graph take turns.  B200, one net's image of 65,536
+// vertices: 0.56 -> 0.08 ms against an allocation per call and two pageable
+// copies.
 void fetch_images(bfx_workspace* ws, std::initializer_list<HostImage> images) {
   struct Piece {
     const char* device;
     char* host;
     size_t bytes;
   };
+  BFX_CUDA(cudaStreamSynchronize(ws->stream));
+  std::lock_guard<std::mutex> lock(ws->graph->image_mutex);
   std::vector<Piece> pieces;
   for (const HostImage& im : images) {
-    if (im.host == nullptr) continue;
+    if (im.host == nullptr || im.bytes == 0) continue;
+    char* const host = static_cast<char*>(im.host);
+    if (known_memory(host, im.bytes)) {
+      BFX_CUDA(cudaMemcpyAsync(host, im.device, im.bytes, cudaMemcpyDeviceToHost, ws->stream));
+      continue;
+    }
     for (size_t at = 0; at < im.bytes; at += kPieceBytes) {
-      pieces.push_back({static_cast<const char*>(im.device) + at, static_cast<char*>(im.host) + at,
-                        std::min(kPieceBytes, im.bytes - at)});
+      pieces.push_back({static_cast<const char*>(im.device) + at, host + at, std::min(kPieceBytes, im.bytes - at)});
     }
   }
   const unsigned threads =
       pieces.size() < 4 ? 1U : std::min<unsigned>({kPieceThreads, std::max(1U, std::thread::hardware_concurrency()),
                                                    static_cast<unsigned>(pieces.size())});
-  BFX_CUDA(cudaStreamSynchronize(ws->stream));
-  std::lock_guard<std::mutex> lock(ws->graph->image_mutex);
   char* const buffer = static_cast<char*>(ws->graph->image_host.ptr);
   std::atomic<size_t> next{0};
   std::atomic<int> error{cudaSuccess};
