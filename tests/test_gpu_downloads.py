@@ -1,4 +1,7 @@
-"""Downloads into page-locked and partly page-locked memory."""
+"""Downloads into page-locked and partly page-locked memory, and from several
+workspaces of one graph at once, on a thread each."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -41,4 +44,60 @@ def test_page_locked_outputs(gpu, locked):
     np.testing.assert_array_equal(got[0].reshape(bits.shape), bits)
     np.testing.assert_array_equal(got[1].reshape(pred.shape), pred)
     ws.close()
+    resident.close()
+
+
+def test_workspaces_on_threads(gpu):
+    """Four workspaces of one graph, each on its own thread and stream: regional
+    sets (clusters), a whole-graph set (a team each), label images of many
+    pieces and paths, all at once, with the results of one after another."""
+    spec = dict(workloads.GRAPHS["c1f"])
+    spec.update(tiles_x=160, tiles_y=160, nodes_per_tile=45)
+    g, order, _ = bfx.synth_graph(**spec)
+    layout = bfx.build_device_graph_layout(g, order)
+    grid = (160, 160)
+    regional = bfx.BatchPlannerPolicy(32, 1, 8, 2, 1, narrow_lanes=True)
+    sets = []
+    for k in range(4):
+        if k == 3:
+            queries = workloads.full_graph_queries(layout, grid, 3, 9, targets_per_query=5)
+            policy = bfx.BatchPlannerPolicy(32, 0, 1, 10000, 1, narrow_lanes=True)
+        else:
+            queries = workloads.box_queries(layout, grid, 24, 2, 40, seed=k, targets=(1, 4))
+            policy = regional
+        sets.append(bfx.make_overlapping_batch_plan(layout, queries, policy).descriptions())
+    resident = bfx.ResidentDeviceGraph.upload_once(layout)
+
+    def one_pass(ws, descs):
+        ws.prepare(descs)
+        ws.execute(bfx.GpuRunOptions())
+        assert all(s.stop_reason == bfx.STOP_CONVERGED for s in ws.fetch_statuses())
+        paths = ws.compact_paths(raw=True)
+        return [*ws.download_lane(0, 0), *ws.download_labels(len(descs) - 1, descs[-1].lane_width),
+                paths["vertices"], paths["labels"], paths["edges"], ws.label_bounds()]
+
+    alone = []
+    for descs in sets:
+        ws = bfx.Workspace(resident)
+        alone.append(one_pass(ws, descs))
+        ws.close()
+    failures, start = [], threading.Barrier(4)
+
+    def worker(k):
+        try:
+            ws = bfx.Workspace(resident)
+            start.wait(60)
+            for _ in range(6):
+                for x, y in zip(one_pass(ws, sets[k]), alone[k], strict=True):
+                    np.testing.assert_array_equal(x, y)
+            ws.close()
+        except BaseException as e:  # noqa: BLE001 -- reported by the test
+            failures.append((k, e))
+
+    threads = [threading.Thread(target=worker, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(120)
+    assert not failures, failures
     resident.close()
