@@ -1403,7 +1403,12 @@ int bfx_workspace_stream(bfx_workspace* ws, void** stream) {
 int bfx_workspace_bytes(bfx_workspace* ws, uint64_t* bytes) {
   return bfx::guarded([&] {
     bfx::require(ws && bytes, "null argument");
-    *bytes = ws->meta.bytes + ws->arena.bytes + ws->tile_tables.bytes + ws->qimage.bytes;
+    *bytes = 0;
+    for (const bfx::DeviceBuffer* b : {&ws->meta, &ws->arena, &ws->tile_tables, &ws->qimage, &ws->image, &ws->paths,
+                                       &ws->adjoint, &ws->mappings_dev, &ws->deltas_dev, &ws->engines_dev,
+                                       &ws->round_trace}) {
+      *bytes += b->bytes;
+    }
   });
 }
 

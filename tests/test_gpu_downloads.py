@@ -101,3 +101,25 @@ def test_workspaces_on_threads(gpu):
         t.join(120)
     assert not failures, failures
     resident.close()
+
+
+def test_workspace_counts_its_buffers(gpu):
+    """The buffers that a workspace keeps from one call to the next are in its
+    reported bytes: the image buffer, the path buffer, the adjoint's."""
+    layout, grid = workloads.build_graph("c1")
+    desc = bfx.make_description(layout, workloads.full_graph_queries(layout, grid, 8, 3), 8)
+    resident = bfx.ResidentDeviceGraph.upload_once(layout)
+    ws = bfx.Workspace(resident)
+    ws.prepare([desc])
+    ws.execute(bfx.GpuRunOptions())
+    held = [ws.device_bytes()]
+    bits, _ = ws.download_labels(0, 8)
+    held.append(ws.device_bytes())
+    targets = len(ws.compact_paths())
+    held.append(ws.device_bytes())
+    ws.edge_usage_adjoint(np.ones(targets, np.float32))
+    held.append(ws.device_bytes())
+    grown = np.diff(held)
+    assert grown[0] >= bits.nbytes and grown[1] >= targets * 28 and grown[2] >= layout.edge_count * 4
+    ws.close()
+    resident.close()
