@@ -656,10 +656,13 @@ int bfx_compact_path_payload(bfx_workspace* ws, uint32_t* vertices, float* dista
     bfx::require(vertices && distance_labels && (edge_ids || ws->path_edges == 0), "null output");
     BFX_CUDA(cudaSetDevice(ws->graph->device));
     const std::uint64_t T = ws->path_targets, nv = ws->path_vertices, ne = ws->path_edges;
-    // Output arena: vertices, labels, edges, kept in the workspace.
+    // Output arena: vertices, labels, edges, kept in the workspace up to the
+    // size of its download buffer, else allocated for the call.
     const size_t out_bytes = bfx::align256(nv * 4) * 2 + bfx::align256(ne * 4 + 4);
-    ws->image.reserve(out_bytes, ws->graph->device);
-    char* const dout = static_cast<char*>(ws->image.ptr);
+    bfx::DeviceBuffer once;
+    bfx::DeviceBuffer& out = out_bytes <= bfx::kImageBytes ? ws->image : once;
+    out.reserve(out_bytes, ws->graph->device);
+    char* const dout = static_cast<char*>(out.ptr);
     bfx::PathArgs a = bfx::path_args(ws);
     a.out_vertices = reinterpret_cast<std::uint32_t*>(dout);
     a.out_labels = reinterpret_cast<float*>(dout + bfx::align256(nv * 4));

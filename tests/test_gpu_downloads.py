@@ -123,3 +123,34 @@ def test_workspace_counts_its_buffers(gpu):
     assert grown[0] >= bits.nbytes and grown[1] >= targets * 28 and grown[2] >= layout.edge_count * 4
     ws.close()
     resident.close()
+
+
+def test_large_payload_is_not_kept(gpu):
+    """6.7 million path vertices (80 MB): the payload's buffer is the call's
+    own, a small one stays with the workspace."""
+    n, targets = 22_400, 300
+    i = np.arange(n)
+    e = n - 1
+    g = bfx.InputGraph(i // 128, np.zeros(n), np.ones(n), np.zeros(n), i[:-1], i[1:], np.ones(e), np.zeros(e),
+                       np.zeros(e), np.arange(e))
+    layout = bfx.build_device_graph_layout(g, bfx.SpatialOrderConfig(0, 0, 1, 1))
+    order = np.argsort(layout.tiles["new_to_old"])
+    resident = bfx.ResidentDeviceGraph.upload_once(layout)
+    ws = bfx.Workspace(resident)
+    for count in (3, targets):
+        q = bfx.RouteQuery(1, [int(order[0])], [int(v) for v in order[n - count:]], np.arange(layout.tile_count))
+        ws.prepare([bfx.make_description(layout, [q], 1)])
+        ws.execute(bfx.GpuRunOptions())
+        before = ws.device_bytes()
+        paths = ws.compact_paths(raw=True)
+        lengths = paths["summaries"]["path_length"].astype(np.int64)
+        assert sorted(lengths) == list(range(n - count, n))
+        ends = np.cumsum(lengths + 1)
+        np.testing.assert_array_equal(paths["labels"][ends - 1], lengths)
+        np.testing.assert_array_equal(paths["vertices"][:lengths[0] + 1], order[:lengths[0] + 1])
+        kept = ws.device_bytes() - before
+        # the path buffer holds the targets' trails and the search's scratch
+        if count == targets:
+            assert len(paths["vertices"]) * 12 > 64 << 20 and kept < 16 << 20
+    ws.close()
+    resident.close()
