@@ -307,7 +307,7 @@ __global__ void init_kernel(LaunchParams p) {
     p.run->sync.abort = 0u;
     p.run->round = 0u;
     p.run->done = 0u;
-    p.run->stop = 0u;
+    p.run->open = 0u;
     p.run->abort = 0u;
     p.run->started = dev::global_ns();
     for (int i = 0; i < 16; ++i) p.run->work[i] = 0u;
@@ -1406,7 +1406,7 @@ int bfx_workspace_bytes(bfx_workspace* ws, uint64_t* bytes) {
     *bytes = 0;
     for (const bfx::DeviceBuffer* b : {&ws->meta, &ws->arena, &ws->tile_tables, &ws->qimage, &ws->image, &ws->paths,
                                        &ws->adjoint, &ws->mappings_dev, &ws->deltas_dev, &ws->engines_dev,
-                                       &ws->round_trace}) {
+                                       &ws->round_trace, &ws->progress}) {
       *bytes += b->bytes;
     }
   });
@@ -2170,6 +2170,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
   const size_t smem = (size_t{ws->nb} + 1) * 4;
   std::uint64_t launches = 0;
   ws->last_host_checks = 0;
+  const auto poll_start = std::chrono::steady_clock::now();
   BFX_CUDA(cudaEventRecord(ws->ev[0], ws->stream));
   // init + seed with a wide ordinary grid
   const int wide = ws->sm_count * 8;
@@ -2219,9 +2220,11 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
                           : (chunked ? reinterpret_cast<const void*>(round_kernel<false, true>)
                                      : reinterpret_cast<const void*>(round_kernel<false, false>));
     const int grid = grid_blocks(ws, kfn, block, smem, o);
-    start_kernel<<<1, 1024, smem, ws->stream>>>(p);
-    ++launches;
-    BFX_CUDA(cudaGetLastError());
+    if (remaining) {
+      start_kernel<<<1, 1024, smem, ws->stream>>>(p);
+      ++launches;
+      BFX_CUDA(cudaGetLastError());
+    }
     // Capture K x (round, advance) once per workspace generation / K / engine.
     const bool reuse = ws->chunk_exec && ws->chunk_rounds == K && ws->chunk_grid == grid &&
                        ws->chunk_instr == o.instrumentation &&
@@ -2263,13 +2266,12 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
     std::uint32_t* const done_host = static_cast<std::uint32_t*>(ws->status_host.ptr);
     const std::uint64_t max_chunks = (o.maximum_rounds + K - 1) / K + 1;
     ws->last_host_checks = 0;
-    const auto t0 = std::chrono::steady_clock::now();
-    for (std::uint64_t c = 0; c < max_chunks; ++c) {
+    for (std::uint64_t c = 0; remaining && c < max_chunks; ++c) {
       BFX_CUDA(cudaMemcpyAsync(done_host, &p.run->done, 4, cudaMemcpyDeviceToHost, ws->stream));
       BFX_CUDA(cudaStreamSynchronize(ws->stream));
       ++ws->last_host_checks;
       if (*done_host) break;
-      if (std::chrono::steady_clock::now() - t0 > std::chrono::nanoseconds(ws->budget_ns)) {
+      if (std::chrono::steady_clock::now() - poll_start > std::chrono::nanoseconds(ws->budget_ns)) {
         // same outcome as a persistent launch past its budget: device_failure
         BFX_CUDA(cudaMemsetAsync(&p.run->abort, 1, 1, ws->stream));
         break;
@@ -2278,9 +2280,11 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
       launches += 2ull * K;
     }
   }
-  if (resident) {
-    launches += launch_teams(ws, p, o.instrumentation != 0u);
-    launches += launch_resident(ws, p, o.instrumentation != 0u);
+  if (resident && o.control_mode == BFX_CONTROL_PERSISTENT_COOPERATIVE) {
+    launches += launch_searches(ws, p, o.instrumentation != 0u);
+  } else if (resident) {
+    const std::uint32_t K = o.control_mode == BFX_CONTROL_PER_ROUND_HOST_POLL ? 1u : o.rounds_per_chunk;
+    launches += poll_searches(ws, p, o.instrumentation != 0u, K, poll_start + std::chrono::nanoseconds(ws->budget_ns));
   }
   BFX_CUDA(cudaGetLastError());
   BFX_CUDA(cudaEventRecord(ws->ev[2], ws->stream));

@@ -105,7 +105,7 @@ struct DRun {
   dev::GridSync sync;
   u32 round;       // next round (host-poll modes)
   u32 done;        // all batches stopped
-  u32 stop;        // launch-wide stop reason
+  u32 open;        // host-poll modes: a search outside the grid-wide kernels has rounds left (resident.cu)
   u32 abort;       // device failure seen
   u64 started;     // %globaltimer when the relaxation began: what its searches' budget counts from
   u64 work[16];    // launch-wide work counters: [0..6] push engines, [7] rounds, [8..11] Jacobi, [12..13] splits,
@@ -200,6 +200,14 @@ struct TeamState {
   u32 reserved[51];
 };
 constexpr u32 kMaxTeams = 8u;
+
+// A search between the launches of a host-polled run (resident.cu).  Clusters:
+// its scalars, `done` once it has converged.  Teams: those of the lane under
+// way (`begun`), after `turns` finished lanes.
+struct SearchProgress {
+  u32 rounds, tau, delta, splits;
+  u32 begun, turns, done, reserved;
+};
 
 constexpr u32 kRoundTraceCap = 65536;
 
@@ -347,6 +355,7 @@ struct bfx_workspace {
   const bfx::u32* d_fit{nullptr};
   std::uint64_t search_rounds{0};    // no search of the prepared set takes more rounds (at least its largest lane's vertices)
   std::uint32_t resident_mode = 1;   // see bfx_set_resident_nets
+  bfx::DeviceBuffer progress;        // host-poll modes: SearchProgress [kMaxTeams], then one per entry of `nets`
   std::uint64_t budget_ns = bfx::kLaunchBudgetNs;  // see bfx_set_launch_budget
   cudaEvent_t resident_fork{nullptr};
   std::vector<bfx::SideStreams<bfx::CudaStreams>::Side> resident_sides;

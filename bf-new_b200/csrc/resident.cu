@@ -27,6 +27,12 @@
 // among the admitted in-edges that give the vertex's distance -- what the
 // packed 64-bit minimum of the other frontier kernels ends in.
 //
+// Host-polled runs (kPolled) launch a search for a chunk of rounds at a time.
+// Between the launches its distances are in the label rows, without
+// predecessors, its pending and far bitmaps in the lane's part of the second
+// label slot (8 bytes a vertex of the union, so 8 a word fit), and its scalars
+// in a SearchProgress.
+//
 // A round of a full block (49 K vertices) costs about 6 us -- two dependent
 // global reads (row, records), the list of pending vertices, the barrier --
 // plus 0.55 ns per relaxed edge (1 ns in a cluster of 8, where a fifth of the
@@ -38,7 +44,7 @@
 // 4,096 vertices 0.26 -> 0.12 ms.
 #include "resident.cuh"
 
-#include <type_traits>
+#include <cstddef>
 
 namespace bfx {
 namespace {
@@ -252,10 +258,11 @@ struct Place {
 
 // kCluster: the net's words are dealt to several blocks (ctas > 1).  kWhole:
 // every tile is one run of words, so it lies in one block and its distances
-// are contiguous there.
-template <bool kCount, bool kCluster, bool kWhole>
+// are contiguous there.  kPolled: at most `chunk` rounds.
+template <bool kCount, bool kCluster, bool kWhole, bool kPolled>
 __global__ void __launch_bounds__(1024, 1)
-    resident_kernel(LaunchParams p, const ResidentNet* nets, u32 cluster_ctas, u32 run) {
+    resident_kernel(LaunchParams p, const ResidentNet* nets, u32 cluster_ctas, u32 run, SearchProgress* progress,
+                    u32 chunk) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ NetShared s;
   const u32 ctas = kCluster ? cluster_ctas : 1u;
@@ -264,7 +271,15 @@ __global__ void __launch_bounds__(1024, 1)
   const u32 rank = kCluster ? cluster_rank() : 0u;
   // uniform over the cluster
   if (engine_of(p, b) != BFX_ENGINE_FRONTIER_PUSH) return;
+  SearchProgress was{};  // written at the end of an earlier launch
+  if (kPolled) {
+    was = progress[blockIdx.x / ctas];
+    if (was.done != 0u) return;
+  }
+  const bool resumed = kPolled && was.rounds != 0u;
   const DBatch& B = p.batches[b];
+  u32* const saved_near = reinterpret_cast<u32*>(B.dist[1] + static_cast<u64>(B.U) * ql);  // by the net's words
+  u32* const saved_far = saved_near + net.words;
   DCtl& C = p.ctl[b];
   const u32 T = p.g.T, dw = (T + 31u) >> 5;
   const u32 M = block_words(net.words, ctas, run);  // words of this block
@@ -348,10 +363,21 @@ __global__ void __launch_bounds__(1024, 1)
       for (u32 k = 0; k * 32u < end - begin; ++k) {
         const Place at = place((word + k) * 32u);
         if (at.owner != rank) continue;
-        if (k * 32u + lane < end - begin) L[at.slot + lane] = dev::kInfBits;
+        if (k * 32u + lane < end - begin) {
+          u32 d = dev::kInfBits;
+          if (resumed) {
+            const u32 cv = begin + k * 32u + lane - B.tiles[tile].y;
+            d = dev::hi(B.dist[0][(static_cast<u64>(cv) << B.shift) + ql]);
+          }
+          L[at.slot + lane] = d;
+        }
         if (lane == 0u) {
           gbase[at.slot >> 5] = begin + k * 32u;
           gtile[at.slot >> 5] = tile;
+          if (resumed) {
+            ((was.rounds & 1u) ? near1 : near0)[at.slot >> 5] = saved_near[word + k];
+            far[at.slot >> 5] = saved_far[word + k];
+          }
         }
       }
     }
@@ -374,7 +400,7 @@ __global__ void __launch_bounds__(1024, 1)
   const u32 near0_off = M * 128u;  // offsets from L
   // --- sources ---------------------------------------------------------------
   const u32 src0 = B.src_off[ql], src1 = B.src_off[ql + 1u];
-  for (u32 i = src0 + tid; i < src1; i += blockDim.x) {
+  for (u32 i = resumed ? src1 : src0 + tid; i < src1; i += blockDim.x) {
     const u32 v = B.src[i], t = p.g.owner[v];
     if (((dir[t >> 5].x >> (t & 31u)) & 1u) == 0u) continue;  // reported by the seed kernel
     const Endpoint e = endpoint(make_uint4(v, 0u, 0u, t));
@@ -386,11 +412,35 @@ __global__ void __launch_bounds__(1024, 1)
   // --- rounds ------------------------------------------------------------------
   u32 delta = p.deltas ? p.deltas[b] : p.auto_step;
   u32 tau = delta, splits = 0u, rounds = 0u, pass = 0u;
+  if (resumed) {
+    delta = was.delta;
+    tau = was.tau;
+    splits = was.splits;
+    rounds = was.rounds;
+  }
+  bool paused = false;
   u32 cnt[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
   u64 total_cnt[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
   for (;; ++rounds) {
     u32* const cur = (rounds & 1u) ? near1 : near0;
     u32* const nxt = (rounds & 1u) ? near0 : near1;
+    if (kPolled && rounds - was.rounds == chunk) {
+      // after a barrier, so no neighbour changes this block's words any more
+      for (u32 w = warp; w < M; w += warps) {
+        const u32 of = kCluster ? ((((w >> run) * ctas + rank) << run) | (w & run_mask)) : w;  // the net's word
+        const u32 d = L[w * 32u + lane];
+        if (d != kPad) {
+          const u32 cv = gbase[w] + lane - B.tiles[gtile[w]].y;
+          B.dist[0][(static_cast<u64>(cv) << B.shift) + ql] = (static_cast<u64>(d) << 32) | kFull;
+        }
+        if (lane == 0u && of < net.words) {
+          saved_near[of] = cur[w];
+          saved_far[of] = far[w];
+        }
+      }
+      paused = true;
+      break;
+    }
     const u32 nxt_off = near0_off + ((rounds & 1u) ? 0u : M * 4u), far_off = near0_off + M * 8u;
     bool any = false;
 
@@ -589,7 +639,7 @@ __global__ void __launch_bounds__(1024, 1)
     }
     cluster_sync(ctas);
   }
-  ++rounds;  // rounds run
+  if (!paused) ++rounds;  // rounds run
 
   // --- result: distances and predecessors -------------------------------------
   // After the last barrier no block changes its distances.  A warp takes a
@@ -597,7 +647,7 @@ __global__ void __launch_bounds__(1024, 1)
   // the vertex's predecessor in shared memory, where the list was.
   __syncthreads();
   volatile u32* const best = reinterpret_cast<u32*>(list) + warp * 32u;
-  for (u32 w = warp; w < M; w += warps) {
+  for (u32 w = paused ? M : warp; w < M; w += warps) {
     const u32 d = L[w * 32u + lane];
     const bool act = d < dev::kInfBits;
     if (!__any_sync(kFull, act)) continue;
@@ -664,6 +714,10 @@ __global__ void __launch_bounds__(1024, 1)
   if (tid == 0u && rank == 0u) {
     atomicMax(&C.rounds, rounds);
     atomicMax(reinterpret_cast<unsigned long long*>(&p.run->work[7]), static_cast<unsigned long long>(rounds));
+    if (kPolled) {
+      progress[blockIdx.x / ctas] = SearchProgress{rounds, tau, delta, splits, 0u, 0u, paused ? 0u : 1u, 0u};
+      if (paused) atomicExch(&p.run->open, 1u);
+    }
   }
   if (kCount) {
     for (int i = 0; i < 7; ++i) {
@@ -707,9 +761,10 @@ __device__ __forceinline__ LaneScratch lane_scratch(const DBatch& B, u32 V, u32 
 
 constexpr u32 kTeamList = 4096u;  // pending vertices of a block's pass
 
-template <bool kCount>
+template <bool kCount, bool kPolled>
 __global__ void __launch_bounds__(1024, 1)
-    team_kernel(LaunchParams p, const ResidentNet* nets, u32 net_count, u32 teams, TeamState* states) {
+    team_kernel(LaunchParams p, const ResidentNet* nets, u32 net_count, u32 teams, TeamState* states,
+                SearchProgress* progress, u32 chunk) {
   __shared__ u32 s_list[kTeamList];
   __shared__ u32 s_listed[2], s_cut[2], s_min[32];
   const u32 per = gridDim.x / teams, team = blockIdx.x / per, rank = blockIdx.x - team * per;
@@ -729,28 +784,48 @@ __global__ void __launch_bounds__(1024, 1)
     if (tid == 0u) atomicExch(&p.run->abort, 1u);
     return false;
   };
-  for (u32 n = team; n < net_count; n += teams) {
+  SearchProgress was{};  // written at the end of an earlier launch
+  if (kPolled) was = progress[team];
+  u32 turn = was.turns, ran = 0u;
+  bool paused = false;
+  for (u32 n = team + turn * teams; n < net_count && !paused; n += teams, ++turn) {
     const u32 b = nets[n].batch, ql = nets[n].lane;
     if (engine_of(p, b) != BFX_ENGINE_FRONTIER_PUSH) continue;
     const DBatch& B = p.batches[b];
     DCtl& C = p.ctl[b];
     const LaneScratch m = lane_scratch(B, V, ql);
     const u64 at = static_cast<u64>(rank) * blockDim.x + tid, stride = static_cast<u64>(per) * blockDim.x;
-    for (u64 i = at; i < V; i += stride) m.L[i] = dev::kInfBits;
-    for (u64 i = at; i < 3ull * words; i += stride) m.near0[i] = 0u;
-    if (!barrier()) return;
-    if (rank == 0u) {
-      for (u32 i = B.src_off[ql] + tid; i < B.src_off[ql + 1u]; i += blockDim.x) {
-        const u32 v = B.src[i];
-        m.L[v] = 0u;
-        dev::red_or(m.near0 + (v >> 5), 1u << (v & 31u));
+    const bool resumed = kPolled && was.begun != 0u && turn == was.turns;
+    if (!resumed) {
+      for (u64 i = at; i < V; i += stride) m.L[i] = dev::kInfBits;
+      for (u64 i = at; i < 3ull * words; i += stride) m.near0[i] = 0u;
+      if (!barrier()) return;
+      if (rank == 0u) {
+        for (u32 i = B.src_off[ql] + tid; i < B.src_off[ql + 1u]; i += blockDim.x) {
+          const u32 v = B.src[i];
+          m.L[v] = 0u;
+          dev::red_or(m.near0 + (v >> 5), 1u << (v & 31u));
+        }
       }
+      if (!barrier()) return;
     }
-    if (!barrier()) return;
     u32 delta = p.deltas ? p.deltas[b] : p.auto_step;
-    u32 tau = delta, rounds = 0u;
-    const u32 splits0 = splits;
-    for (;; ++rounds) {
+    u32 tau = delta, rounds = 0u, splits0 = splits;
+    if (resumed) {
+      delta = was.delta;
+      tau = was.tau;
+      rounds = was.rounds;
+      splits0 -= was.splits;
+    }
+    for (;; ++rounds, ++ran) {
+      if (kPolled && ran == chunk) {  // after a barrier: the lane's scratch is whole
+        if (rank == 0u && tid == 0u) {
+          progress[team] = SearchProgress{rounds, tau, delta, splits - splits0, 1u, turn, 0u, 0u};
+          atomicExch(&p.run->open, 1u);
+        }
+        paused = true;
+        break;
+      }
       u32* const cur = (rounds & 1u) ? m.near1 : m.near0;
       u32* const nxt = (rounds & 1u) ? m.near0 : m.near1;
       bool any = false;
@@ -932,10 +1007,15 @@ __global__ void __launch_bounds__(1024, 1)
       }
       if (converged) break;
     }
+    const u32 run_rounds = paused ? rounds : rounds + 1u;
+    if (!paused) ++ran;
     if (tid == 0u && rank == 0u) {
-      atomicMax(&C.rounds, rounds + 1u);
-      atomicMax(reinterpret_cast<unsigned long long*>(&p.run->work[7]), static_cast<unsigned long long>(rounds + 1u));
+      atomicMax(&C.rounds, run_rounds);
+      atomicMax(reinterpret_cast<unsigned long long*>(&p.run->work[7]), static_cast<unsigned long long>(run_rounds));
     }
+  }
+  if (kPolled && !paused && turn != was.turns && rank == 0u && tid == 0u) {
+    progress[team] = SearchProgress{0u, 0u, 0u, 0u, 0u, turn, 1u, 0u};
   }
   if (kCount) {
     for (int i = 0; i < 7; ++i) {
@@ -1069,21 +1149,23 @@ __global__ void __launch_bounds__(256) team_predecessor_kernel(LaunchParams p, u
   }
 }
 
-const void* team_entry(bool count) {
-  return count ? reinterpret_cast<const void*>(team_kernel<true>) : reinterpret_cast<const void*>(team_kernel<false>);
+template <bool kCount>
+const void* team_entry(bool polled) {
+  return polled ? reinterpret_cast<const void*>(team_kernel<kCount, true>)
+                : reinterpret_cast<const void*>(team_kernel<kCount, false>);
 }
 
-const void* resident_entry(bool count, bool cluster, bool whole) {
-  if (!cluster) {  // one block: a tile is contiguous in any case
-    return count ? reinterpret_cast<const void*>(resident_kernel<true, false, true>)
-                 : reinterpret_cast<const void*>(resident_kernel<false, false, true>);
-  }
-  if (whole) {
-    return count ? reinterpret_cast<const void*>(resident_kernel<true, true, true>)
-                 : reinterpret_cast<const void*>(resident_kernel<false, true, true>);
-  }
-  return count ? reinterpret_cast<const void*>(resident_kernel<true, true, false>)
-               : reinterpret_cast<const void*>(resident_kernel<false, true, false>);
+// (one block: a tile is contiguous in any case)
+template <bool kCount, bool kPolled>
+const void* resident_entry(bool cluster, bool whole) {
+  if (!cluster) return reinterpret_cast<const void*>(resident_kernel<kCount, false, true, kPolled>);
+  return whole ? reinterpret_cast<const void*>(resident_kernel<kCount, true, true, kPolled>)
+               : reinterpret_cast<const void*>(resident_kernel<kCount, true, false, kPolled>);
+}
+
+const void* resident_entry(bool count, bool polled, bool cluster, bool whole) {
+  if (count) return polled ? resident_entry<true, true>(cluster, whole) : resident_entry<true, false>(cluster, whole);
+  return polled ? resident_entry<false, true>(cluster, whole) : resident_entry<false, false>(cluster, whole);
 }
 
 }  // namespace
@@ -1121,10 +1203,12 @@ void set_attributes(const void* kernel) {
 // largest cluster that it can hold at once.  Sets the kernels' attributes,
 // which hold for the device, so that launches need not.
 u32 resident_shapes() {
-  for (int count = 0; count < 2; ++count) {
-    for (int kind = 0; kind < 3; ++kind) set_attributes(resident_entry(count != 0, kind != 0, kind == 2));
+  for (int k = 0; k < 4; ++k) {
+    for (int kind = 0; kind < 3; ++kind) {
+      set_attributes(resident_entry((k & 1) != 0, (k & 2) != 0, kind != 0, kind == 2));
+    }
   }
-  const void* kernel = resident_entry(false, true, true);
+  const void* kernel = resident_entry(false, false, true, true);
   u32 shapes = 1u;
   for (; shapes < kShapeCount; ++shapes) {
     if (kShapes[shapes].ctas == 1u) continue;
@@ -1173,7 +1257,10 @@ void resident_select(bfx_workspace* ws, const std::vector<u32>& full, std::vecto
   });
 }
 
-u32 launch_teams(bfx_workspace* ws, const LaunchParams& p, bool count) {
+namespace {
+
+// Launches the whole-graph lanes' searches.
+u32 launch_teams(bfx_workspace* ws, const LaunchParams& p, bool count, SearchProgress* progress, u32 chunk) {
   if (ws->whole.empty()) return 0;
   // Lanes at a time: as many as kTeamBytes of distances allow, in equal turns.
   // More teams hide one another's barriers and read latency, until their wave
@@ -1190,24 +1277,31 @@ u32 launch_teams(bfx_workspace* ws, const LaunchParams& p, bool count) {
   TeamState* states = ws->d_teams;
   BFX_CUDA(cudaMemsetAsync(states, 0, sizeof(TeamState) * kMaxTeams, ws->stream));
   LaunchParams params = p;
-  void* args[] = {&params, &d_whole, &lanes, &teams, &states};
-  BFX_CUDA(cudaLaunchCooperativeKernel(team_entry(count), dim3(static_cast<u32>(ws->sm_count) / teams * teams),
-                                       dim3(1024), args, 0, ws->stream));
-  u32 launches = 1;
-  for (u32 i = 0, last = 0xFFFFFFFFu; i < lanes; ++i) {
-    const u32 b = ws->whole[i].batch;
-    if (b == last) continue;
-    last = b;
-    team_rows_kernel<<<ws->sm_count * 6, 256, 0, ws->stream>>>(params, b);
+  void* args[] = {&params, &d_whole, &lanes, &teams, &states, &progress, &chunk};
+  const void* kernel = count ? team_entry<true>(progress != nullptr) : team_entry<false>(progress != nullptr);
+  BFX_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(static_cast<u32>(ws->sm_count) / teams * teams), dim3(1024), args,
+                                       0, ws->stream));
+  return 1;
+}
+
+// Label rows and predecessors of the whole-graph lanes.
+u32 launch_team_labels(bfx_workspace* ws, const LaunchParams& p) {
+  u32 launches = 0;
+  u32 last = 0xFFFFFFFFu;
+  for (const ResidentNet& n : ws->whole) {
+    if (n.batch == last) continue;
+    last = n.batch;
+    team_rows_kernel<<<ws->sm_count * 6, 256, 0, ws->stream>>>(p, n.batch);
     BFX_CUDA(cudaGetLastError());
-    team_predecessor_kernel<<<ws->sm_count * 8, 256, 0, ws->stream>>>(params, b);
+    team_predecessor_kernel<<<ws->sm_count * 8, 256, 0, ws->stream>>>(p, n.batch);
     BFX_CUDA(cudaGetLastError());
     launches += 2;
   }
   return launches;
 }
 
-u32 launch_resident(bfx_workspace* ws, const LaunchParams& p, bool count) {
+// Launches the searches of the nets that have clusters of their own.
+u32 launch_resident(bfx_workspace* ws, const LaunchParams& p, bool count, SearchProgress* progress, u32 chunk) {
   const std::vector<ResidentNet>& nets = ws->nets;
   if (nets.empty()) return 0;
   const u32 run = ws->graph->word_run;
@@ -1278,13 +1372,53 @@ u32 launch_resident(bfx_workspace* ws, const LaunchParams& p, bool count) {
     LaunchParams params = p;
     const ResidentNet* d_nets = ws->d_nets + first;
     u32 ctas = sh.ctas, run_shift = run;
-    void* args[] = {&params, &d_nets, &ctas, &run_shift};
-    const void* kernel = resident_entry(count, sh.ctas > 1u, ws->graph->word_whole);
+    SearchProgress* net_progress = progress ? progress + first : nullptr;
+    void* args[] = {&params, &d_nets, &ctas, &run_shift, &net_progress, &chunk};
+    const void* kernel = resident_entry(count, progress != nullptr, sh.ctas > 1u, ws->graph->word_whole);
     BFX_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
     ++launches;
   }
   sides.join();
   return launches;
+}
+
+}  // namespace
+
+u32 launch_searches(bfx_workspace* ws, const LaunchParams& p, bool count) {
+  u32 launches = launch_teams(ws, p, count, nullptr, 0u) + launch_team_labels(ws, p);
+  launches += launch_resident(ws, p, count, nullptr, 0u);
+  return launches;
+}
+
+// A chunk costs about 0.1 ms beside its rounds (host calls of up to eight
+// streams, the net's tables and distances set up again): 40 nets of 67 rounds,
+// 8 at a time, 1.76 ms a request on a B200, 0.93 in one launch, and 4.7 in the
+// grid-wide rounds.  One graph launch per chunk costs more than it saves
+// (2.2 ms: it is made anew for every prepared set).
+u32 poll_searches(bfx_workspace* ws, const LaunchParams& p, bool count, u32 chunk,
+                  std::chrono::steady_clock::time_point deadline) {
+  const size_t bytes = (kMaxTeams + ws->nets.size()) * sizeof(SearchProgress);
+  ws->progress.reserve(bytes, ws->graph->device);
+  auto* const progress = static_cast<SearchProgress*>(ws->progress.ptr);
+  BFX_CUDA(cudaMemsetAsync(progress, 0, bytes, ws->stream));
+  ws->status_host.reserve(256);
+  auto* const seen = static_cast<u32*>(ws->status_host.ptr);  // {open, abort}
+  static_assert(offsetof(DRun, abort) == offsetof(DRun, open) + 4);
+  u32 launches = 0;
+  for (;;) {
+    BFX_CUDA(cudaMemsetAsync(&p.run->open, 0, 4, ws->stream));
+    launches += launch_teams(ws, p, count, progress, chunk);
+    launches += launch_resident(ws, p, count, progress + kMaxTeams, chunk);
+    BFX_CUDA(cudaMemcpyAsync(seen, &p.run->open, 8, cudaMemcpyDeviceToHost, ws->stream));
+    BFX_CUDA(cudaStreamSynchronize(ws->stream));
+    ++ws->last_host_checks;
+    if (seen[0] == 0u || seen[1] != 0u) break;
+    if (std::chrono::steady_clock::now() > deadline) {
+      BFX_CUDA(cudaMemsetAsync(&p.run->abort, 1, 1, ws->stream));
+      break;
+    }
+  }
+  return launches + launch_team_labels(ws, p);
 }
 
 void resident_release(bfx_workspace* ws) {

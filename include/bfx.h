@@ -361,7 +361,10 @@ int bfx_get_frontier_mapping(bfx_workspace *ws, uint32_t *layout, uint32_t count
  * (each tile rounded up to 32; no search takes more rounds, so none stops on
  * its limit), an explicit grid, round tracing, another frontier layout or an option of the grid-wide kernels (bfx_set_register_budget,
  * _flat_items, _flat_order, _relax_atomic, _chunk_pairs) stay grid-wide.  The
- * round count of a batch is then the largest of its lanes'. */
+ * round count of a batch is then the largest of its lanes'.  In the host-poll
+ * modes a search runs in launches of at most rounds_per_chunk rounds (one, per
+ * round), and the host looks after each whether rounds are left and whether
+ * the budget is spent; bfx_fetch_work_statistics counts those looks. */
 int bfx_set_resident_nets(bfx_workspace *ws, uint32_t mode);
 /* Wall-clock budget of a relaxation, 1 ns .. 30 s (the default).  The kernels
  * look at it every few rounds; a launch past it stops and its batches report
