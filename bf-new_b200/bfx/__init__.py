@@ -800,6 +800,13 @@ class Workspace:
         _check(load().bfx_fetch_work_statistics(self._h, None, out))
         return dict(zip(self.WORK_KEYS, (int(x) for x in out)))
 
+    def last_execute_kernels(self) -> dict:
+        """Kind of kernel ("clusters", "teams", "grid") -> (lanes it relaxed in the last execute, registers per
+        thread; 0 where none ran)."""
+        lanes, regs = (u32 * 3)(), (u32 * 3)()
+        _check(load().bfx_last_execute_kernels(self._h, lanes, regs))
+        return {k: (int(n), int(r)) for k, n, r in zip(("clusters", "teams", "grid"), lanes, regs)}
+
     def round_trace(self) -> np.ndarray:
         """(rounds, 4) array of {start ns, warp items | split batches << 32, active pairs,
         lane-edge relaxations} from the last instrumentation-2 persistent run."""

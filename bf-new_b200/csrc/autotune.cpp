@@ -309,15 +309,17 @@ extern "C" int bfx_autotune(bfx_workspace* ws, uint32_t count, const bfx_batch_d
           if (bfx::time_set(ws, oa, trials) >= t_visits) bfx::check(bfx_set_batch_mappings(ws, 0, nullptr));
         }
       }
-      // Phase 5, in context: chunk slots per warp item, 2, 4 or 8 (the
-      // class's choice when cached).
+      // Phase 5, in context, where lanes are relaxed grid-wide: chunk slots
+      // per warp item, 2, 4 or 8 (the class's choice when cached).
       if (set_cached) {
         pack = set_choice.pack;
         bfx::check(bfx_set_chunk_pack(ws, pack));
       } else {
         float t_best = bfx::time_set(ws, oa, trials);
+        std::uint32_t lanes[3], registers[3];
+        bfx::check(bfx_last_execute_kernels(ws, lanes, registers));
         for (const std::uint32_t k : {2U, 4U, 8U}) {
-          if (k == pack) continue;
+          if (k == pack || lanes[2] == 0U) continue;  // clusters and teams have no chunk slots
           bfx::check(bfx_set_chunk_pack(ws, k));
           const float t = bfx::time_set(ws, oa, trials);
           if (t < t_best) {

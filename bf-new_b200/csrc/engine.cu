@@ -2166,6 +2166,20 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
       remaining = !frontier || (ws->batches[b].valid & ~ws->fit[b]) != 0u;
     }
   }
+  std::uint32_t lanes = 0;
+  std::fill_n(ws->last_lanes, 3, 0U);
+  std::fill_n(ws->last_kernels, 3, nullptr);
+  for (const DBatch& b : ws->batches) lanes += static_cast<std::uint32_t>(__builtin_popcount(b.valid));
+  if (resident) {
+    const auto count = [&](const std::vector<ResidentNet>& searches) {
+      return static_cast<std::uint32_t>(std::count_if(searches.begin(), searches.end(), [&](const ResidentNet& n) {
+        return p.engines == nullptr || ws->engines_uploaded[n.batch] == BFX_ENGINE_FRONTIER_PUSH;
+      }));
+    };
+    ws->last_lanes[0] = count(ws->nets);
+    ws->last_lanes[1] = count(ws->whole);
+  }
+  ws->last_lanes[2] = lanes - ws->last_lanes[0] - ws->last_lanes[1];
   const int block = static_cast<int>(o.block_size);
   const size_t smem = (size_t{ws->nb} + 1) * 4;
   std::uint64_t launches = 0;
@@ -2195,6 +2209,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
     const int grid = grid_blocks(ws, kfn, block, tsmem, o);
     void* args[] = {&p};
     BFX_CUDA(cudaLaunchCooperativeKernel(kfn, grid, block, args, tsmem, ws->stream));
+    ws->last_kernels[2] = kfn;
     ++launches;
   } else if (o.control_mode == BFX_CONTROL_PERSISTENT_COOPERATIVE) {
     // register budget 0 (default): 80 for the chunked layout with blocks of
@@ -2209,6 +2224,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
     if (remaining) {
       void* args[] = {&p};
       BFX_CUDA(cudaLaunchCooperativeKernel(kfn, grid, block, args, smem, ws->stream));
+      ws->last_kernels[2] = kfn;
       ++launches;
     }
   } else {
@@ -2221,6 +2237,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
                                      : reinterpret_cast<const void*>(round_kernel<false, false>));
     const int grid = grid_blocks(ws, kfn, block, smem, o);
     if (remaining) {
+      ws->last_kernels[2] = kfn;
       start_kernel<<<1, 1024, smem, ws->stream>>>(p);
       ++launches;
       BFX_CUDA(cudaGetLastError());
@@ -2516,6 +2533,20 @@ int bfx_fetch_label_bounds(bfx_workspace* ws, uint32_t* max_finite_distance_bits
     bfx::label_bound_kernel<<<ws->sm_count * 8, 256, 0, ws->stream>>>(ws->params, ws->d_status, d_out);
     BFX_CUDA(cudaGetLastError());
     bfx::fetch_images(ws, {{d_out, max_finite_distance_bits, bytes}});
+  });
+}
+
+int bfx_last_execute_kernels(bfx_workspace* ws, uint32_t lanes[3], uint32_t registers[3]) {
+  return bfx::guarded([&] {
+    bfx::require(ws && lanes && registers, "null argument");
+    bfx::require(ws->executed, "no executed batches");
+    BFX_CUDA(cudaSetDevice(ws->graph->device));
+    for (int k = 0; k < 3; ++k) {
+      cudaFuncAttributes a{};
+      if (ws->last_kernels[k]) BFX_CUDA(cudaFuncGetAttributes(&a, ws->last_kernels[k]));
+      lanes[k] = ws->last_lanes[k];
+      registers[k] = static_cast<std::uint32_t>(a.numRegs);
+    }
   });
 }
 

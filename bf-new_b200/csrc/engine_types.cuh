@@ -324,6 +324,9 @@ struct bfx_workspace {
   bfx_device_controller* d_ctrl{nullptr};
   std::uint64_t last_launches{0};
   std::uint64_t last_host_checks{0};
+  // Kernels of the last execute (bfx_last_execute_kernels): clusters, teams, grid-wide.
+  std::uint32_t last_lanes[3] = {0, 0, 0};
+  const void* last_kernels[3] = {nullptr, nullptr, nullptr};
   std::uint64_t last_h2d{0}, last_d2h{0};
   cudaEvent_t ev[4]{};  // execute start, relaxation start, relaxation end, execute end
   bool executed{false};

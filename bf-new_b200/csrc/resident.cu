@@ -1281,6 +1281,7 @@ u32 launch_teams(bfx_workspace* ws, const LaunchParams& p, bool count, SearchPro
   const void* kernel = count ? team_entry<true>(progress != nullptr) : team_entry<false>(progress != nullptr);
   BFX_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(static_cast<u32>(ws->sm_count) / teams * teams), dim3(1024), args,
                                        0, ws->stream));
+  ws->last_kernels[1] = kernel;
   return 1;
 }
 
@@ -1376,6 +1377,7 @@ u32 launch_resident(bfx_workspace* ws, const LaunchParams& p, bool count, Search
     void* args[] = {&params, &d_nets, &ctas, &run_shift, &net_progress, &chunk};
     const void* kernel = resident_entry(count, progress != nullptr, sh.ctas > 1u, ws->graph->word_whole);
     BFX_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+    if (i == 0) ws->last_kernels[0] = kernel;
     ++launches;
   }
   sides.join();

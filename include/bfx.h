@@ -289,8 +289,9 @@ int bfx_resident_graph_set_weights(bfx_resident_graph *graph, const float *weigh
  * each batch shape's dense rounds are mapped to tile visits or chunk-slot
  * warp items (timed alone, visits where 1.1x faster, cached per shape), the
  * per-batch mix kept only if the whole set runs faster (bfx_get_frontier_mapping
- * reports the outcome); last, 2, 4 and 8 chunk slots per warp item are timed
- * on the whole set and the fastest kept (bfx_get_chunk_pack reports it).  The
+ * reports the outcome); last, where lanes take the grid-wide kernels, 2, 4 and
+ * 8 chunk slots per warp item are timed on the whole set and the fastest kept
+ * (bfx_get_chunk_pack reports it).  The
  * step, layout and pack are cached per set class (graph, magnitudes of the
  * batch counts per lane width and of the union size) and reused for a later
  * set of the class.  Leaves the workspace prepared with all `count`
@@ -419,6 +420,12 @@ int bfx_barrier_selftest(int device, uint32_t rounds, uint32_t absent_block, uin
 
 /* Kernels launched by the most recent bfx_execute (its own kernels only). */
 int bfx_last_launch_count(bfx_workspace *ws, uint64_t *launches);
+
+/* What relaxed the lanes of the most recent bfx_execute: lanes searched by
+ * clusters, by teams of blocks and by the grid-wide kernels
+ * (bfx_set_resident_nets), and the registers per thread of each kind's kernel
+ * (clusters: of the largest shape; 0 where none was launched). */
+int bfx_last_execute_kernels(bfx_workspace *ws, uint32_t lanes[3], uint32_t registers[3]);
 
 /* Work counters of the most recent bfx_execute run with instrumentation >= 1
  * (the reference's Light level, gpu_api.hpp:40-44): stats in the reference's
