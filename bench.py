@@ -7,7 +7,9 @@ Workload (default c2): 128x128 tiles x 128 nodes (2,097,152 vertices,
 16,777,216 edges), float costs base(span) * lognormal(0, 0.5); 256 regional
 queries with box sides U[4,64] tiles, one source and one target each; the
 planner groups overlapping queries into batches (narrowed to 1/8/16/32
-lanes) and one persistent cooperative launch relaxes all of them.  On one GPU
+lanes), and one execute relaxes all of them: lanes that fit a thread-block
+cluster in clusters side by side, larger whole-graph lanes by teams of blocks,
+the rest in one persistent cooperative launch.  On one GPU
 the default run also times c3 (64 full-graph sources on 256x256 tiles x 256
 nodes, 16.8M V / 168M E, uint costs) and c5 (4,096 regional + 16 full-graph
 queries on the same graph) and reports them in the line's `c3` and `c5`
@@ -54,8 +56,8 @@ for _p in (REPO, REPO / "bf-new_b200"):
 import numpy as np  # noqa: E402
 
 METRICS = {
-    "c2": "batched SSSP queries/s (256 uneven regional queries, 2.1M V / 16.8M E, one persistent launch)",
-    "c3": "batched SSSP queries/s (64 full-graph sources, 16.8M V / 168M E, one persistent launch)",
+    "c2": "batched SSSP queries/s (256 uneven regional queries, 2.1M V / 16.8M E)",
+    "c3": "batched SSSP queries/s (64 full-graph sources, 16.8M V / 168M E)",
     "c5": "batched SSSP queries/s (4,096 regional + 16 full-graph queries, 16.8M V / 168M E, autotuned)",
     "c3small": "batched SSSP queries/s (32 full-graph sources, 4.2M V / 42M E, profiling-sized c3)",
 }
@@ -108,6 +110,24 @@ def traffic_estimate(workload: str, relaxations: int, kernel_ms: float, step: st
         random_ceiling = {"dram_gbs": dram_gbs, "peak_gbs": ceiling[0] / 1e9, "frac": dram_gbs * 1e9 / ceiling[0],
                           "source": ceiling[1] + " (random 32-byte sectors beyond the L2)"}
     return traffic, source, random_ceiling
+
+
+def roofline_bytes(workload: str, kernels: dict, alg_bytes: int, relaxations: int, kernel_ms: float, step: str,
+                   layout: str, search_path: Path | None = None):
+    """What a launch moves through DRAM, for the roofline: (bytes or None, what they are,
+    traffic, its source, the random-sector ceiling).  The algorithmic bytes count the grid-wide
+    kernels' reads and writes, so they describe a launch only where no lane was searched by
+    clusters or teams; their distances live in shared memory and the L2.  Sets searched by
+    clusters alone have captures of their own (profiles/search_traffic.txt)."""
+    if kernels["clusters"][0] == 0 and kernels["teams"][0] == 0:
+        if layout != "chunked":  # the committed traffic captures are of the chunked kernel
+            return alg_bytes, "algorithmic bytes", None, f"no capture of the {layout} kernel is scaled", None
+        return alg_bytes, "algorithmic bytes", *traffic_estimate(workload, relaxations, kernel_ms, step)
+    if kernels["teams"][0] or kernels["grid"][0] or workload != "c2":
+        return None, "not defined", None, "no capture of these cluster, team and grid-wide lanes is scaled", None
+    path = search_path or REPO / "profiles" / "search_traffic.txt"
+    traffic, source, _ = traffic_estimate(workload, relaxations, kernel_ms, step, path)
+    return traffic, "DRAM bytes, scaled from a capture" if traffic else "not defined", traffic, source, None
 
 
 def step_label(engines, deltas, mean_weight: float) -> str:
@@ -311,13 +331,8 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
                   "tiled": bfx.FRONTIER_TILED}
     ws.set_frontier_layout(layout_ids[args.frontier])
     ws.set_register_budget(args.regs)
-    eff_regs = args.regs or (80 if args.frontier == "chunked" else 64)
-    if args.frontier != "chunked" and eff_regs == 80:
-        eff_regs = 64
-    if args.frontier == "tiled":
-        eff_regs = 128  # the tiled kernel's own bound: two 256-thread blocks per SM
-        if args.stage_min is not None:
-            ws.set_tile_stage_min(args.stage_min)
+    if args.frontier == "tiled" and args.stage_min is not None:
+        ws.set_tile_stage_min(args.stage_min)
     ws.set_flat_items(args.items)
     ws.set_relax_atomic(args.amin)
     ws.set_flat_order(args.edge_major)
@@ -355,8 +370,6 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
     layout_names = {v: k for k, v in layout_ids.items()}
     tuned_layout, tuned_mappings = ws.frontier_mapping(len(descs))
     frontier_used = layout_names[tuned_layout]
-    if frontier_used == "tiled":
-        eff_regs = 128
     opts = bfx.GpuRunOptions(engine=engine_id)
     opts_instr = bfx.GpuRunOptions(engine=engine_id, instrumentation=1)
 
@@ -411,6 +424,7 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
         kernel_ms.append(k)
         execute_ms.append(x)
     launches_per_step = ws.last_launch_count()
+    kernels = ws.last_execute_kernels()
     dev_ms = max_over_ranks(dev_ms)
     log(f"[bench] {wl.name} device-resident: {dev_ms / steps:.3f} ms/step, relaxation kernel "
         f"{np.mean(kernel_ms):.3f} ms")
@@ -501,19 +515,13 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
         peak_src = "measured"
     else:
         peak, peak_src = 6650.0, "fallback"
-    achieved = alg_bytes / (kernel_avg / 1000) / 1e9
     engines_for_step = engines_chosen or [2 if engine_id == bfx.ENGINE_FRONTIER_PUSH else engine_id] * len(descs)
     step = step_label(engines_for_step, deltas, mean_w)
-    # the library's defaults relax lanes in clusters and teams of blocks; the
-    # grid-wide chunked kernel runs where an option of its own is set
-    off_grid = (frontier_used == "chunked" and args.regs == 0 and args.items == 2 and not args.amin
-                and not args.edge_major and not args.pairs)
-    if off_grid:
-        traffic, traffic_source, random_ceiling = None, "no capture of the cluster and team kernels is scaled", None
-    elif frontier_used == "chunked":
-        traffic, traffic_source, random_ceiling = traffic_estimate(wl.name, work["relaxations"], kernel_avg, step)
-    else:  # the committed traffic captures are of the chunked kernel
-        traffic, traffic_source, random_ceiling = None, f"no capture of the {frontier_used} kernel is scaled", None
+    moved, moved_what, traffic, traffic_source, random_ceiling = roofline_bytes(
+        wl.name, kernels, alg_bytes, work["relaxations"], kernel_avg, step, frontier_used)
+    achieved = moved / (kernel_avg / 1000) / 1e9 if moved else None
+    grid_name = "persistent_tiled_kernel" if frontier_used == "tiled" else "persistent_kernel"
+    kernel_names = {"clusters": "resident_kernel", "teams": "team_kernel", "grid": grid_name}
     line = {
         "metric": METRICS[wl.name], "value": value, "unit": "queries/s", "n_gpus": world, "steps": steps,
         "warmup": warmup, "ms_per_step": ms_per_step, "higher_is_better": True,
@@ -529,7 +537,8 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
                    "frontier_layout": frontier_used,
                    "tile_visit_batches": (sum(1 for m in tuned_mappings if m == bfx.MAPPING_TILE_VISITS)
                                           if frontier_used == "tiled" else 0),
-                   "registers": 64 if off_grid else eff_regs, "flat_items": args.items,
+                   "lanes": {k: n for k, (n, _) in kernels.items()},
+                   "registers": {kernel_names[k]: r for k, (n, r) in kernels.items() if n}, "flat_items": args.items,
                    "returning_min": args.amin, "edge_major": args.edge_major, "chunk_pairs": args.pairs,
                    "chunk_pack": ws.chunk_pack(),
                    "engines_chosen": None if engines_chosen is None else
@@ -545,15 +554,16 @@ def measure(wl, args, *, rank, world, dist, device, steps, warmup, shard=False, 
         "host": {"plan_s": plan_s, "tune_s": tune_s,
                  "note": "host planner (batch grouping + descriptions) and autotuner run once per query set, "
                          "before both timed regions"},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+        "roofline": {"bound": "hbm" if kernels["grid"][0] else "dependent rounds (shared memory, L2 and barriers)",
+                     "achieved": achieved, "achieved_is": moved_what, "peak": peak, "unit": "GB/s",
+                     "frac": achieved / peak if achieved else None,
                      "traffic": traffic, "traffic_source": traffic_source, "peak_source": peak_src,
-                     "random_sector_ceiling": random_ceiling, "kernel": "%s (%s frontier, %d registers%s)" % (
-                         "resident_kernel and team_kernel" if off_grid else
-                         "persistent_tiled_kernel" if frontier_used == "tiled" else "persistent_kernel",
-                         frontier_used, 64 if off_grid else eff_regs,
+                     "random_sector_ceiling": random_ceiling, "kernel": " and ".join(
+                         f"{kernel_names[k]} ({n} lanes, {r} registers)" for k, (n, r) in kernels.items() if n) + (
                          ", mixed engines" if engines_chosen and any(e != 2 for e in engines_chosen) else ""),
                      "kernel_ms": kernel_avg, "execute_ms": float(np.mean(execute_ms)),
-                     "algorithmic_bytes_per_launch": alg_bytes, "work": work, "engine_work": engine_work},
+                     "algorithmic_bytes_per_launch": alg_bytes if moved_what == "algorithmic bytes" else None,
+                     "work": work, "engine_work": engine_work},
         "clocks": clocks.summary(),
         "gpu_launches": launches_per_step * steps,
     }
