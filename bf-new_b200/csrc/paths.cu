@@ -739,12 +739,15 @@ extern "C" int bfx_resident_graph_set_weights(bfx_resident_graph* graph, const f
     bfx::require(graph && weights_by_edge_id, "null argument");
     const std::uint32_t E = graph->g.E;
     std::vector<float> w(weights_by_edge_id, weights_by_edge_id + E);
-    for (float& x : w) {
+    double sums[8] = {};  // eight chains: one addition waits for the last of its own
+    for (std::uint32_t i = 0; i < E; ++i) {
+      float& x = w[i];
       if (!(x >= 0.0f) || x == __builtin_inff()) throw std::invalid_argument("edge weights must be finite and nonnegative");
       if (x == 0.0f) x = 0.0f;  // canonical +0 (InputGraph canonicalisation)
+      sums[i & 7u] += x;
     }
     double sum = 0.0;
-    for (const float x : w) sum += x;
+    for (const double x : sums) sum += x;
     BFX_CUDA(cudaSetDevice(graph->device));
     float* d = nullptr;
     BFX_CUDA(cudaMalloc(reinterpret_cast<void**>(&d), size_t{E} * 4 + 4));
