@@ -49,7 +49,7 @@ def test_page_locked_outputs(gpu, locked):
 
 def test_workspaces_on_threads(gpu):
     """Four workspaces of one graph, each on its own thread and stream: regional
-    sets (clusters), a whole-graph set (a team each), label images of many
+    sets (clusters), whole-graph sets (a team each), label images of many
     pieces and paths, all at once, with the results of one after another."""
     spec = dict(workloads.GRAPHS["c1f"])
     spec.update(tiles_x=160, tiles_y=160, nodes_per_tile=45)
@@ -59,8 +59,8 @@ def test_workspaces_on_threads(gpu):
     regional = bfx.BatchPlannerPolicy(32, 1, 8, 2, 1, narrow_lanes=True)
     sets = []
     for k in range(4):
-        if k == 3:
-            queries = workloads.full_graph_queries(layout, grid, 3, 9, targets_per_query=5)
+        if k >= 2:
+            queries = workloads.full_graph_queries(layout, grid, 3, 9 + k, targets_per_query=5)
             policy = bfx.BatchPlannerPolicy(32, 0, 1, 10000, 1, narrow_lanes=True)
         else:
             queries = workloads.box_queries(layout, grid, 24, 2, 40, seed=k, targets=(1, 4))
