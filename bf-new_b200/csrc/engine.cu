@@ -2484,7 +2484,7 @@ int bfx_download_labels(bfx_workspace* ws, uint32_t batch, uint32_t* distance_bi
     // vertex ranges of at most kImageBytes, so that the buffer stays small
     const std::uint32_t V = ws->graph->g.V;
     const std::uint32_t rows = static_cast<std::uint32_t>(std::min<size_t>(V, bfx::kImageBytes / (size_t{8} << B.shift)));
-    ws->image.reserve((size_t{rows} << B.shift) * 8, ws->graph->device);
+    ws->image.reserve_pooled((size_t{rows} << B.shift) * 8, ws->graph->device, ws->stream);
     for (std::uint32_t v0 = 0; v0 < V; v0 += rows) {
       const size_t n = size_t{std::min(rows, V - v0)} << B.shift, at = size_t{v0} << B.shift;
       auto* d_out = static_cast<std::uint32_t*>(ws->image.ptr);
@@ -2508,7 +2508,7 @@ int bfx_download_lane_labels(bfx_workspace* ws, uint32_t batch, uint32_t lane, u
     BFX_CUDA(cudaSetDevice(ws->graph->device));
     const std::uint32_t V = ws->graph->g.V;
     const std::uint32_t rows = static_cast<std::uint32_t>(std::min<size_t>(V, bfx::kImageBytes / 8));
-    ws->image.reserve(size_t{rows} * 8, ws->graph->device);
+    ws->image.reserve_pooled(size_t{rows} * 8, ws->graph->device, ws->stream);
     for (std::uint32_t v0 = 0; v0 < V; v0 += rows) {
       const std::uint32_t n = std::min(rows, V - v0);
       auto* d_out = static_cast<std::uint32_t*>(ws->image.ptr);
@@ -2527,7 +2527,7 @@ int bfx_fetch_label_bounds(bfx_workspace* ws, uint32_t* max_finite_distance_bits
     bfx::require(ws->executed, "no executed batches");
     BFX_CUDA(cudaSetDevice(ws->graph->device));
     const size_t bytes = size_t{ws->nb} * 4;
-    ws->image.reserve(bytes, ws->graph->device);
+    ws->image.reserve_pooled(bytes, ws->graph->device, ws->stream);
     auto* d_out = static_cast<std::uint32_t*>(ws->image.ptr);
     BFX_CUDA(cudaMemsetAsync(d_out, 0, bytes, ws->stream));
     bfx::label_bound_kernel<<<ws->sm_count * 8, 256, 0, ws->stream>>>(ws->params, ws->d_status, d_out);

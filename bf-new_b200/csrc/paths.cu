@@ -660,9 +660,13 @@ int bfx_compact_path_payload(bfx_workspace* ws, uint32_t* vertices, float* dista
     // size of its download buffer, else allocated for the call.
     const size_t out_bytes = bfx::align256(nv * 4) * 2 + bfx::align256(ne * 4 + 4);
     bfx::DeviceBuffer once;
-    bfx::DeviceBuffer& out = out_bytes <= bfx::kImageBytes ? ws->image : once;
-    out.reserve(out_bytes, ws->graph->device);
-    char* const dout = static_cast<char*>(out.ptr);
+    const bool kept = out_bytes <= bfx::kImageBytes;
+    if (kept) {
+      ws->image.reserve_pooled(out_bytes, ws->graph->device, ws->stream);
+    } else {
+      once.reserve(out_bytes, ws->graph->device);
+    }
+    char* const dout = static_cast<char*>((kept ? ws->image : once).ptr);
     bfx::PathArgs a = bfx::path_args(ws);
     a.out_vertices = reinterpret_cast<std::uint32_t*>(dout);
     a.out_labels = reinterpret_cast<float*>(dout + bfx::align256(nv * 4));
