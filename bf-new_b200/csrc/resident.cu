@@ -36,12 +36,14 @@
 // A round of a full block (49 K vertices) costs about 6 us -- two dependent
 // global reads (row, records), the list of pending vertices, the barrier --
 // plus 0.55 ns per relaxed edge (1 ns in a cluster of 8, where a fifth of the
-// targets are in other blocks).  Rows are read as one list of edges per 32
-// vertices: with 2 or 4 threads per row the loads' partial lines bounded the
-// launch (B200, 256 regional nets, 2.1 M vertices: 12.4 and 10.6 ms against
-// 10.5).  Relaxation launch of that set 22.6 -> 10.6 ms; 512 nets on 65 K vertices
-// 7.8 -> 1.7 ms; 8 whole images of 65 K vertices 2.18 -> 0.66 ms; one net of
-// 4,096 vertices 0.26 -> 0.12 ms.
+// targets are in other blocks).  Neither DRAM (15 % of its rate) nor the L2
+// (3 %) bounds it: a warp waits at the round's barriers, then for the records.
+// Rows are read as one list of edges per 32 vertices: with 2 or 4 threads per row the
+// loads' partial lines bounded the launch (B200, 256 regional nets, 2.1 M
+// vertices, when measured: 12.4 and 10.6 ms against 10.5).  Relaxation launch of
+// that set 22.6 -> 10.2 ms; 512 nets on 65 K vertices 7.8 -> 1.7 ms; 8 whole
+// images of 65 K vertices 2.18 -> 0.47 ms; one net of 4,096 vertices 0.26 ->
+// 0.11 ms.
 #include "resident.cuh"
 
 #include <cstddef>

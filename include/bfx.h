@@ -224,7 +224,7 @@ int bfx_fetch_label_bounds(bfx_workspace *ws, uint32_t *max_finite_distance_bits
 
 /* Device time of the most recent bfx_execute, measured by CUDA events the
  * library records on the workspace stream: out[0] = relaxation kernels
- * (the persistent launch, or all round/advance launches of a host-poll run),
+ * (searches and the persistent launch, or all launches of a host-poll run),
  * out[1] = the whole execute (init, seed, relaxation, finalize), in ms. */
 int bfx_last_execute_timing(bfx_workspace *ws, float out[2]);
 /* Bytes moved by the most recent bfx_prepare_batches (H2D) and
@@ -432,7 +432,8 @@ int bfx_last_execute_kernels(bfx_workspace *ws, uint32_t lanes[3], uint32_t regi
  * DeviceWorkStatistics layout; counters (may be NULL) = {queue entries
  * processed, edge records read, active (vertex, lane) source reads, lane-edge
  * relaxations, queue claims, distance decreases, min-reductions issued,
- * rounds}.  Without instrumentation the counters read zero. */
+ * rounds}.  Lanes searched by clusters and teams count no queue claims.
+ * Without instrumentation the counters read zero. */
 int bfx_fetch_work_statistics(bfx_workspace *ws, bfx_device_work_statistics *stats, uint64_t counters[8]);
 /* The same counters split by engine (bfx extension, for per-engine
  * algorithmic byte counts): [0..6] frontier and dense push in the order

@@ -210,7 +210,7 @@ struct BatchedCompactPathOutput {
 };
 
 // One engine kind behind bf-new's batched-engine calls.  Every call relaxes
-// its batch set in one persistent launch on the engine's own stream; calls
+// its batch set in one bfx_execute on the engine's own stream; calls
 // must be sequential (as for the HIP engines).  Non-owning: the resident
 // graph must outlive the engine.
 template <EngineKind kKind>
