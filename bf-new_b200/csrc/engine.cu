@@ -1456,7 +1456,7 @@ Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector
   const size_t o_status = align256(o_sbase + (count + 1) * 4);
   const size_t o_ctrl = align256(o_status + count * sizeof(bfx_device_run_status));
   const size_t o_fit = align256(o_ctrl + count * sizeof(bfx_device_controller));
-  const size_t o_nets = align256(o_fit + count * 4);
+  const size_t o_nets = align256(o_fit + count * 8);
   Layout L;
   const size_t o_whole = align256(o_nets + nets.size() * sizeof(ResidentNet));
   const size_t o_teams = align256(o_whole + whole.size() * sizeof(ResidentNet));
@@ -1566,13 +1566,18 @@ Layout lay_out_batches(bfx_workspace* ws, std::uint32_t count, const std::vector
   sbase[count] = static_cast<std::uint32_t>(ssum);
   ws->search_rounds = whole.empty() ? 0u : g.V;
   if (!nets.empty()) ws->search_rounds = std::max(ws->search_rounds, u64{nets[0].words} * 32u);  // largest first
-  for (const ResidentNet& n : whole) ws->batches[n.batch].team = 1u;
+  ws->fit_teams.assign(count, 0u);
+  for (const ResidentNet& n : whole) {
+    ws->batches[n.batch].team = 1u;
+    ws->fit_teams[n.batch] |= 1u << n.lane;
+  }
   std::memcpy(hb + o_batch, ws->batches.data(), count * sizeof(DBatch));
   if (!whole.empty()) std::memcpy(hb + o_whole, whole.data(), whole.size() * sizeof(ResidentNet));
   ws->whole.swap(whole);
   ws->d_whole = reinterpret_cast<const ResidentNet*>(db + o_whole);
   ws->d_teams = reinterpret_cast<TeamState*>(db + o_teams);
   std::memcpy(hb + o_fit, fit.data(), count * 4);
+  std::memcpy(hb + o_fit + count * 4, ws->fit_teams.data(), count * 4);
   if (!nets.empty()) std::memcpy(hb + o_nets, nets.data(), nets.size() * sizeof(ResidentNet));
   ws->fit.swap(fit);
   ws->nets.swap(nets);
@@ -2153,17 +2158,22 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
   // (resident.cu); what remains takes the grid-wide kernels.  Not for launches
   // that may stop on their round limit (kLateRounds), that trace rounds, or
   // that set a grid, a layout or an option of the grid-wide kernels.
-  const bool resident = ws->resident_mode != 0u && !(ws->nets.empty() && ws->whole.empty()) && p.flat == 2u &&
+  const std::uint32_t poll_rounds = o.control_mode == BFX_CONTROL_PERSISTENT_COOPERATIVE ? 0u
+                                    : o.control_mode == BFX_CONTROL_PER_ROUND_HOST_POLL ? 1u
+                                                                                        : o.rounds_per_chunk;
+  const bool clusters = !ws->nets.empty() && (poll_rounds == 0u || poll_rounds >= kPolledClusterRounds);
+  const bool resident = ws->resident_mode != 0u && (clusters || !ws->whole.empty()) && p.flat == 2u &&
                         ws->frontier_layout == BFX_FRONTIER_CHUNKED && p.engine == BFX_ENGINE_FRONTIER_PUSH &&
                         o.maximum_rounds >= std::max(kLateRounds, ws->search_rounds) && o.instrumentation < 2u &&
                         o.grid_policy == 0u && ws->relax_atomic == 0u && ws->edge_major == 0u &&
                         ws->chunk_pairs == 0u && ws->flat_items == 2u && ws->register_budget == 0u;
   bool remaining = !resident;
   if (resident) {
-    p.fit = ws->d_fit;
+    const std::vector<std::uint32_t>& fit = clusters ? ws->fit : ws->fit_teams;
+    p.fit = clusters ? ws->d_fit : ws->d_fit + ws->nb;
     for (std::uint32_t b = 0; b < ws->nb && !remaining; ++b) {
       const bool frontier = p.engines == nullptr || ws->engines_uploaded[b] == BFX_ENGINE_FRONTIER_PUSH;
-      remaining = !frontier || (ws->batches[b].valid & ~ws->fit[b]) != 0u;
+      remaining = !frontier || (ws->batches[b].valid & ~fit[b]) != 0u;
     }
   }
   std::uint32_t lanes = 0;
@@ -2176,7 +2186,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
         return p.engines == nullptr || ws->engines_uploaded[n.batch] == BFX_ENGINE_FRONTIER_PUSH;
       }));
     };
-    ws->last_lanes[0] = count(ws->nets);
+    ws->last_lanes[0] = clusters ? count(ws->nets) : 0u;
     ws->last_lanes[1] = count(ws->whole);
   }
   ws->last_lanes[2] = lanes - ws->last_lanes[0] - ws->last_lanes[1];
@@ -2228,7 +2238,7 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
       ++launches;
     }
   } else {
-    const std::uint32_t K = o.control_mode == BFX_CONTROL_PER_ROUND_HOST_POLL ? 1u : o.rounds_per_chunk;
+    const std::uint32_t K = poll_rounds;
     const bool chunked = p.flat == 2u;
     const void* kfn = o.instrumentation
                           ? (chunked ? reinterpret_cast<const void*>(round_kernel<true, true>)
@@ -2300,8 +2310,8 @@ void execute(bfx_workspace* ws, const bfx_gpu_run_options& o) {
   if (resident && o.control_mode == BFX_CONTROL_PERSISTENT_COOPERATIVE) {
     launches += launch_searches(ws, p, o.instrumentation != 0u);
   } else if (resident) {
-    const std::uint32_t K = o.control_mode == BFX_CONTROL_PER_ROUND_HOST_POLL ? 1u : o.rounds_per_chunk;
-    launches += poll_searches(ws, p, o.instrumentation != 0u, K, poll_start + std::chrono::nanoseconds(ws->budget_ns));
+    launches += poll_searches(ws, p, o.instrumentation != 0u, clusters, poll_rounds,
+                              poll_start + std::chrono::nanoseconds(ws->budget_ns));
   }
   BFX_CUDA(cudaGetLastError());
   BFX_CUDA(cudaEventRecord(ws->ev[2], ws->stream));

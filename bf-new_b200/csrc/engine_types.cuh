@@ -146,6 +146,16 @@ constexpr u64 kLaunchBudgetNs = 30000000000ull;   // 30 s per relaxation: all la
 // from this limit on.
 constexpr u64 kLateRounds = 65536u;
 
+// Host-polled runs with fewer rounds a launch keep the lanes that fit a cluster
+// on the grid, where a round is two launches of a captured graph: a cluster
+// sets its tables and distances up again in every launch.  B200, 40 nets on
+// 152K vertices, grid / clusters at 1, 2, 3, 4 and 8 rounds a launch: 4.5 / 8.4,
+// 4.2 / 4.7, 4.1 / 3.4, 4.0 / 2.7, 3.9 / 1.6 ms; 200 nets there 8.8 / 24.9, 8.5 /
+// 13.5, 8.4 / 9.4, 8.4 / 7.4, 8.3 / 4.3; 8 nets on 2.1M vertices 2.5 / 5.3, 2.3 /
+// 3.2, 2.2 / 2.4, 2.2 / 1.9, 2.1 / 1.4.  Teams are faster from one round on (24
+// lanes of 2.1M vertices 92 / 27 ms).
+constexpr u32 kPolledClusterRounds = 4u;
+
 // Near/far step of a set that was given none, in mean edge weights.  Plain
 // frontiers (one round per hop) relax 2.5 to 3 times as many edges as steps of
 // 4 on the regional and whole-graph configurations; steps of 2 to 8 are within
@@ -364,7 +374,7 @@ struct bfx_workspace {
   // Cluster-resident searches (resident.cu): the lanes that fit a cluster,
   // largest first, and per batch the mask of those lanes; host and device.
   std::vector<bfx::ResidentNet> nets, whole;  // whole: whole-graph lanes that no cluster holds
-  std::vector<std::uint32_t> fit;
+  std::vector<std::uint32_t> fit, fit_teams;  // fit_teams: the lanes of `whole` alone; on the device behind `fit`
   const bfx::ResidentNet* d_nets{nullptr};
   const bfx::ResidentNet* d_whole{nullptr};
   bfx::TeamState* d_teams{nullptr};

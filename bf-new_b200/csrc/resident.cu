@@ -1399,7 +1399,7 @@ u32 launch_searches(bfx_workspace* ws, const LaunchParams& p, bool count) {
 // 8 at a time, 1.76 ms a request on a B200, 0.93 in one launch, and 4.7 in the
 // grid-wide rounds.  One graph launch per chunk costs more than it saves
 // (2.2 ms: it is made anew for every prepared set).
-u32 poll_searches(bfx_workspace* ws, const LaunchParams& p, bool count, u32 chunk,
+u32 poll_searches(bfx_workspace* ws, const LaunchParams& p, bool count, bool clusters, u32 chunk,
                   std::chrono::steady_clock::time_point deadline) {
   const size_t bytes = (kMaxTeams + ws->nets.size()) * sizeof(SearchProgress);
   ws->progress.reserve(bytes, ws->graph->device);
@@ -1412,7 +1412,7 @@ u32 poll_searches(bfx_workspace* ws, const LaunchParams& p, bool count, u32 chun
   for (;;) {
     BFX_CUDA(cudaMemsetAsync(&p.run->open, 0, 4, ws->stream));
     launches += launch_teams(ws, p, count, progress, chunk);
-    launches += launch_resident(ws, p, count, progress + kMaxTeams, chunk);
+    if (clusters) launches += launch_resident(ws, p, count, progress + kMaxTeams, chunk);
     BFX_CUDA(cudaMemcpyAsync(seen, &p.run->open, 8, cudaMemcpyDeviceToHost, ws->stream));
     BFX_CUDA(cudaStreamSynchronize(ws->stream));
     ++ws->last_host_checks;

@@ -23,11 +23,11 @@ void resident_select(bfx_workspace* ws, const std::vector<u32>& full, std::vecto
 // launches.
 u32 launch_searches(bfx_workspace* ws, const LaunchParams& p, bool count);
 
-// The same under host control: launches of at most `chunk` rounds, after each
-// of which the host looks whether a search has rounds left (counted in
-// ws->last_host_checks) and, past the deadline, stops the run as a device
-// failure.
-u32 poll_searches(bfx_workspace* ws, const LaunchParams& p, bool count, u32 chunk,
+// The same under host control (the nets only with `clusters`): launches of at
+// most `chunk` rounds, after each of which the host looks whether a search has
+// rounds left (counted in ws->last_host_checks) and, past the deadline, stops
+// the run as a device failure.
+u32 poll_searches(bfx_workspace* ws, const LaunchParams& p, bool count, bool clusters, u32 chunk,
                   std::chrono::steady_clock::time_point deadline);
 
 // Releases the workspace's streams and events of these launches.

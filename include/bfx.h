@@ -365,7 +365,8 @@ int bfx_get_frontier_mapping(bfx_workspace *ws, uint32_t *layout, uint32_t count
  * round count of a batch is then the largest of its lanes'.  In the host-poll
  * modes a search runs in launches of at most rounds_per_chunk rounds (one, per
  * round), and the host looks after each whether rounds are left and whether
- * the budget is spent; bfx_fetch_work_statistics counts those looks. */
+ * the budget is spent; bfx_fetch_work_statistics counts those looks.  With
+ * fewer than four rounds a launch the lanes that fit a cluster stay grid-wide. */
 int bfx_set_resident_nets(bfx_workspace *ws, uint32_t mode);
 /* Wall-clock budget of a relaxation, 1 ns .. 30 s (the default).  The kernels
  * look at it every few rounds; a launch past it stops and its batches report

@@ -33,6 +33,8 @@ def test_lanes_by_kernel(gpu):
     assert used(whole) == (0, 3, 0)
     assert used(regional + whole) == (20, 3, 0)
     assert used(regional + whole, control_mode=bfx.CONTROL_CHUNKED) == (20, 3, 0)
+    assert used(regional + whole, control_mode=bfx.CONTROL_PER_ROUND) == (0, 3, 20)
+    assert used(regional, control_mode=bfx.CONTROL_CHUNKED, rounds_per_chunk=3) == (0, 0, 20)
     assert used(regional + whole, maximum_rounds=60_000) == (0, 0, 23)
     on_grid = sum(bin(d.valid_lane_mask).count("1") for b, d in enumerate(regional) if b % 3 != 2)
     assert used(regional, engine=bfx.ENGINE_AUTO, engines=True) == (20 - on_grid, 0, on_grid)
